@@ -30,3 +30,54 @@ def test_gradient_at_tile_edges(n):
     for a, b in ((mlp_ref.P_W1, mlp_ref.P_B1), (mlp_ref.P_B1, mlp_ref.P_W2), (mlp_ref.P_W2, mlp_ref.P_B2),
                  (mlp_ref.P_B2, mlp_ref.P_W3), (mlp_ref.P_W3, mlp_ref.P_B3), (mlp_ref.P_B3, mlp_ref.P_N)):
         assert np.linalg.norm(g[a:b] - gr[a:b]) <= 2.0 ** -8 * np.linalg.norm(gr[a:b]), (a, b)
+
+
+def _leaves(kind, n):
+    """Chunk ranges over n cubes: a treetop's ascending ones, with gaps and an
+    end beyond the cubes, out of order, overlapping, and with an empty one."""
+    from tgvreconclaude_gb300 import formats as F
+    e = np.linspace(0, n, 8).astype(int)
+    r = {"none": [], "one": [(0, n - 1)], "ascending": [(a, b - 1) for a, b in zip(e, e[1:]) if b > a],
+         "gaps": [(e[1], e[2] - 1), (e[3], e[4] - 1), (e[6], 2 * n + 5)], "reversed": [(e[4], n - 1), (0, e[4] - 1)],
+         "overlap": [(0, e[5]), (e[2], n - 1)], "empty": [(5, 2), (0, n - 1)]}[kind]
+    lv = np.zeros(len(r), F.LEAF_DTYPE)
+    for k, (a, b) in enumerate(r):
+        lv[k] = (k * 0x01000000, k * 0x10000, k % 5, max(0, a), max(0, b))
+    return lv if len(lv) else None
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 256, 257, 5003])
+@pytest.mark.parametrize("kind", ["none", "one", "ascending", "gaps", "reversed", "overlap", "empty"])
+@pytest.mark.parametrize("nbins", [8, 10])
+def test_fused_warm_start_is_features_then_network(n, kind, nbins):
+    """The one-pass warm start equals median + predict(features), bit for bit,
+    whatever the chunk ranges."""
+    from tgvreconclaude_gb300 import scenes as S
+    rng = np.random.default_rng(n)
+    cubes = S.random_octree(rng, 2, 6, n, shape="plane")
+    hists = S.random_histograms(rng, len(cubes), nbins)
+    lv = _leaves(kind, len(cubes))
+    m = WS.WarmStartMLP(nbins, seed=2)
+    y = m.predict(m.features(cubes, hists, lv))
+    assert m.warm_start(cubes, hists, lv).tobytes() == (WS.median_start(hists) + y).astype(np.float32).tobytes()
+
+
+def test_fused_warm_start_takes_rows_at_any_word():
+    """Device histogram rows that start on 4 bytes only (the wide loads need 8 or 16)."""
+    import torch
+    from tgvreconclaude_gb300 import scenes as S
+    rng = np.random.default_rng(1)
+    for nbins in (8, 10):
+        cubes = S.random_octree(rng, 2, 6, 1000)
+        hists = S.random_histograms(rng, len(cubes), nbins)
+        m = WS.WarmStartMLP(nbins, seed=2)
+        want = m.warm_start(cubes, hists)
+        c = torch.from_numpy(cubes.view(np.int32).reshape(-1, 4).copy()).cuda()
+        buf = torch.zeros(hists.size + 1, dtype=torch.int32, device="cuda")
+        buf[1:] = torch.from_numpy(hists.view(np.int32).reshape(-1)).cuda()
+        u = torch.empty(len(cubes), device="cuda")
+        torch.cuda.synchronize()
+        m.ctx.check(m.lib.tgvg_mlp_warm_start_dev(m.ctx.h, m.h, c.data_ptr(), buf[1:].data_ptr(), len(cubes), nbins,
+                                                  None, 0, u.data_ptr()), "warm start")
+        torch.cuda.synchronize()
+        assert u.cpu().numpy().tobytes() == want.tobytes()

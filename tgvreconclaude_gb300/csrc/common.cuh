@@ -151,7 +151,7 @@ enum BufId {
     B_Q1, B_DAT, B_SNAP, B_LID, B_LEAVES, B_ACC, B_FLAGS, B_RANGES, B_RESID, B_LVSTAT,
     B_BARB, B_P4B, B_Q4B, B_Q1B, B_FSLOT, B_FHALO, B_FHCNT,
     // learned warm start
-    B_M_X, B_M_T, B_M_IDX, B_M_Y, B_M_LEAVES, B_M_LEAFID,
+    B_M_X, B_M_T, B_M_IDX, B_M_Y, B_M_LEAVES, B_M_LEAFID, B_M_BOXES,
     // surface extraction
     B_S_CUBES, B_S_STATE, B_S_KEYS, B_S_DEPTH, B_S_U, B_S_HD, B_S_HKEYS, B_S_HMIN, B_S_HMAX, B_S_NBR,
     B_S_FLAGS, B_S_QIDX, B_S_SCAN, B_S_RANK, B_S_LEAF, B_S_QKEY, B_S_QPOS, B_S_QFLIP, B_S_VTK, B_S_VTF,

@@ -84,52 +84,112 @@ __global__ void k_mlp_pack(const float* __restrict__ prm, uint32_t* __restrict__
     frag[t] = pack_bf16(lo, hi);
 }
 
-// Features: bins / total, depth / 21, the position of the cube's centre
-// inside its chunk's node (TreetopLeaf code/depth; the root without leaves) and
-// the median indicator.  `med` (optional) receives the median indicator in
-// FP32 as the reference computes it (src/histogram.cpp:12-31; 0 when empty).
+// A chunk's node as the features need it: the index range of its cubes, the
+// fine-grid coordinates of the node's corner and 1 / its edge (a power of two).
+struct LeafBox {
+    uint32_t first, last;
+    uint32_t x, y, z;
+    float inv_size;
+};
+__host__ __device__ __forceinline__ LeafBox leaf_box(const tgvg_leaf& l) {
+    const uint64_t key = (uint64_t(l.hi) << 32) | l.lo;
+    const int d = l.depth < 0 ? 0 : (l.depth > 21 ? 21 : l.depth);
+    return LeafBox{l.first_idx, l.last_idx, gather3(key), gather3(key >> 1), gather3(key >> 2),
+                   1.0f / (float)(1u << (21 - d))};
+}
+
+// depth / 21 and the median indicator of a first half bin, tabled once per block.
+struct FeatureTables {
+    float depth[22];
+    float med[16];  // [km + 1]; 0: no bin (only a total that wraps 32 bits)
+};
 template <int NB>
-__global__ void k_mlp_features(int n, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
-                               const int* __restrict__ leaf_id, const tgvg_leaf* __restrict__ leaves,
-                               uint32_t* __restrict__ X, float* __restrict__ med) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t* row = hists + (size_t)i * NB;
+__device__ __forceinline__ void feature_tables(FeatureTables& t) {
+    if (threadIdx.x < 22) t.depth[threadIdx.x] = threadIdx.x / 21.0f;
+    if (threadIdx.x <= NB)
+        t.med[threadIdx.x] = fadd(-1.0f, fdiv(fadd((float)((int)threadIdx.x - 1), 0.5f), NB / 2.0f));
+}
+
+// One cube's 16 features as eight bf16 pairs: bins / total, depth / 21, the
+// position of the cube's centre inside its chunk's node (the root without one)
+// and the median indicator, whose FP32 value (the reference's,
+// src/histogram.cpp:12-31; 0 when empty) is returned.  b: the histogram row.
+template <int NB>
+__device__ __forceinline__ float feature_row(const uint32_t (&b)[NB], const uint4& cb, const LeafBox& box,
+                                             const FeatureTables& tab, uint32_t (&out)[8]) {
     float f[MLP_K1];
 #pragma unroll
     for (int k = 0; k < MLP_K1; ++k) f[k] = 0.f;
     uint32_t tot = 0;
 #pragma unroll
-    for (int k = 0; k < NB; ++k) tot += row[k];
+    for (int k = 0; k < NB; ++k) tot += b[k];
     const float inv = tot ? 1.0f / (float)tot : 0.f;
     uint32_t cum = 0;
     int km = -1;
 #pragma unroll
     for (int k = 0; k < NB; ++k) {
-        f[k] = (float)row[k] * inv;
-        cum += row[k];
+        f[k] = (float)b[k] * inv;
+        cum += b[k];
         if (km < 0 && cum * 2 >= tot) km = k;
     }
-    const float m = tot ? fadd(-1.0f, fdiv(fadd((float)km, 0.5f), NB / 2.0f)) : 0.0f;
+    const float m = tot ? tab.med[km + 1] : 0.0f;
     f[NB + 4] = m;
-    if (med) med[i] = m;
-    const uint4 cb = cubes[i];
     const uint64_t key = (uint64_t(cb.x) << 32) | cb.y;
     const int d = min(21, max(0, (int)cb.w));
-    f[NB] = d / 21.0f;
-    uint64_t nkey = 0;
-    int nd = 0;
-    const int l = leaf_id ? leaf_id[i] : -1;
-    if (l >= 0) { nkey = (uint64_t(leaves[l].hi) << 32) | leaves[l].lo; nd = min(21, max(0, leaves[l].depth)); }
-    const float nsize = (float)(1u << (21 - nd)), half = 0.5f * (float)(1u << (21 - d));
-    const uint32_t cx = gather3(key), cy = gather3(key >> 1), cz = gather3(key >> 2);
-    const uint32_t nx = gather3(nkey), ny = gather3(nkey >> 1), nz = gather3(nkey >> 2);
-    f[NB + 1] = fminf(fmaxf(((float)cx - (float)nx + half) / nsize, 0.f), 1.f);
-    f[NB + 2] = fminf(fmaxf(((float)cy - (float)ny + half) / nsize, 0.f), 1.f);
-    f[NB + 3] = fminf(fmaxf(((float)cz - (float)nz + half) / nsize, 0.f), 1.f);
-    uint32_t* out = X + (size_t)i * 8;
+    f[NB] = tab.depth[d];
+    const float half = 0.5f * (float)(1u << (21 - d));
+    // the node's edge is a power of two: the product with its inverse is the quotient
+    f[NB + 1] = fminf(fmaxf(((float)gather3(key) - (float)box.x + half) * box.inv_size, 0.f), 1.f);
+    f[NB + 2] = fminf(fmaxf(((float)gather3(key >> 1) - (float)box.y + half) * box.inv_size, 0.f), 1.f);
+    f[NB + 3] = fminf(fmaxf(((float)gather3(key >> 2) - (float)box.z + half) * box.inv_size, 0.f), 1.f);
 #pragma unroll
     for (int k = 0; k < 8; ++k) out[k] = pack_bf16(f[2 * k], f[2 * k + 1]);
+    return m;
+}
+
+// A histogram row in registers; vec: rows start on 16 (8 bins) or 8 bytes (10 bins).
+template <int NB>
+__device__ __forceinline__ void load_bins(const uint32_t* __restrict__ row, bool vec, uint32_t (&b)[NB]) {
+    if (vec) {
+        if (NB == 8) {
+#pragma unroll
+            for (int k = 0; k < NB; k += 4) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + k));
+                b[k] = v.x; b[k + 1] = v.y; b[k + 2] = v.z; b[k + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NB; k += 2) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + k));
+                b[k] = v.x; b[k + 1] = v.y;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < NB; ++k) b[k] = __ldg(row + k);
+    }
+}
+template <int NB>
+__device__ __forceinline__ bool bins_aligned(const uint32_t* hists) {
+    return ((uintptr_t)hists & (NB == 8 ? 15 : 7)) == 0;
+}
+
+template <int NB>
+__global__ void k_mlp_features(int n, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
+                               const int* __restrict__ leaf_id, const tgvg_leaf* __restrict__ leaves,
+                               uint32_t* __restrict__ X) {
+    __shared__ FeatureTables tab;
+    feature_tables<NB>(tab);
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t b[NB], w[8];
+    load_bins<NB>(hists + (size_t)i * NB, bins_aligned<NB>(hists), b);
+    const int l = leaf_id ? leaf_id[i] : -1;
+    feature_row<NB>(b, cubes[i], leaf_box(l >= 0 ? leaves[l] : tgvg_leaf{0, 0, 0, 0, 0}), tab, w);
+    uint32_t* out = X + (size_t)i * 8;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = w[k];
 }
 
 __global__ void k_leaf_id(int n, int nleaf, const tgvg_leaf* __restrict__ leaves, int* __restrict__ out) {
@@ -141,62 +201,84 @@ __global__ void k_leaf_id(int n, int nleaf, const tgvg_leaf* __restrict__ leaves
     out[i] = id;
 }
 
-// One warp's two hidden layers over a 16-row tile whose input is the A fragment
-// a0..a3: h1 and h2 receive the bf16 activations as the A fragments of the next
-// layer (h[kc][0..3]: rows g / g+8 of columns 16 kc + 2c.., then of 16 kc + 8 + 2c..).
-__device__ __forceinline__ void mlp_hidden(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                           const uint32_t* __restrict__ sfrag, const float* __restrict__ sbias,
-                                           uint32_t (&h)[4][4], uint32_t (&h2)[4][4]) {
+// The first hidden layer over one warp's T 16-row tiles whose inputs are the A
+// fragments a[t]: h receives the bf16 activations as the A fragments of the next
+// layer (h[t][kc][0..3]: rows g / g+8 of columns 16 kc + 2c.., then of
+// 16 kc + 8 + 2c..).  The tiles share the weight fragments' reads.
+template <int T>
+__device__ __forceinline__ void mlp_layer1(const uint32_t (&a)[T][4], const uint32_t* __restrict__ sfrag,
+                                           const float* __restrict__ sbias, uint32_t (&h)[T][4][4]) {
     const int lane = threadIdx.x & 31, c = lane & 3;
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-        const float bl = sbias[nt * 8 + 2 * c], bh = sbias[nt * 8 + 2 * c + 1];
-        float d0 = bl, d1 = bh, d2 = bl, d3 = bh;
-        const uint32_t* bf = sfrag + F_W1 + nt * 64 + lane * 2;
-        mma_bf16(d0, d1, d2, d3, a0, a1, a2, a3, bf[0], bf[1]);
-        d0 = fmaxf(d0, 0.f); d1 = fmaxf(d1, 0.f); d2 = fmaxf(d2, 0.f); d3 = fmaxf(d3, 0.f);
-        const int kc = nt >> 1;
-        if ((nt & 1) == 0) { h[kc][0] = pack_bf16(d0, d1); h[kc][1] = pack_bf16(d2, d3); }
-        else { h[kc][2] = pack_bf16(d0, d1); h[kc][3] = pack_bf16(d2, d3); }
-    }
+        const float2 b = *reinterpret_cast<const float2*>(sbias + nt * 8 + 2 * c);
+        const uint2 w = *reinterpret_cast<const uint2*>(sfrag + F_W1 + nt * 64 + lane * 2);
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-        const float bl = sbias[64 + nt * 8 + 2 * c], bh = sbias[64 + nt * 8 + 2 * c + 1];
-        float d0 = bl, d1 = bh, d2 = bl, d3 = bh;
+        for (int t = 0; t < T; ++t) {
+            float d0 = b.x, d1 = b.y, d2 = b.x, d3 = b.y;
+            mma_bf16(d0, d1, d2, d3, a[t][0], a[t][1], a[t][2], a[t][3], w.x, w.y);
+            h[t][nt >> 1][(nt & 1) * 2] = pack_bf16(fmaxf(d0, 0.f), fmaxf(d1, 0.f));
+            h[t][nt >> 1][(nt & 1) * 2 + 1] = pack_bf16(fmaxf(d2, 0.f), fmaxf(d3, 0.f));
+        }
+    }
+}
+
+// Columns 16 k2 .. 16 k2 + 15 of the second hidden layer: one A fragment per tile.
+template <int T>
+__device__ __forceinline__ void mlp_layer2(int k2, const uint32_t (&h)[T][4][4], const uint32_t* __restrict__ sfrag,
+                                           const float* __restrict__ sbias, uint32_t (&h2)[T][4]) {
+    const int lane = threadIdx.x & 31, c = lane & 3;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int nt = 2 * k2 + half;
+        const float2 b = *reinterpret_cast<const float2*>(sbias + 64 + nt * 8 + 2 * c);
+        float d[T][4];
+#pragma unroll
+        for (int t = 0; t < T; ++t) { d[t][0] = d[t][2] = b.x; d[t][1] = d[t][3] = b.y; }
 #pragma unroll
         for (int kc = 0; kc < 4; ++kc) {
-            const uint32_t* bf = sfrag + F_W2 + (kc * 8 + nt) * 64 + lane * 2;
-            mma_bf16(d0, d1, d2, d3, h[kc][0], h[kc][1], h[kc][2], h[kc][3], bf[0], bf[1]);
+            const uint2 w = *reinterpret_cast<const uint2*>(sfrag + F_W2 + (kc * 8 + nt) * 64 + lane * 2);
+#pragma unroll
+            for (int t = 0; t < T; ++t)
+                mma_bf16(d[t][0], d[t][1], d[t][2], d[t][3], h[t][kc][0], h[t][kc][1], h[t][kc][2], h[t][kc][3], w.x, w.y);
         }
-        d0 = fmaxf(d0, 0.f); d1 = fmaxf(d1, 0.f); d2 = fmaxf(d2, 0.f); d3 = fmaxf(d3, 0.f);
-        const int kc = nt >> 1;
-        if ((nt & 1) == 0) { h2[kc][0] = pack_bf16(d0, d1); h2[kc][1] = pack_bf16(d2, d3); }
-        else { h2[kc][2] = pack_bf16(d0, d1); h2[kc][3] = pack_bf16(d2, d3); }
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            h2[t][half * 2] = pack_bf16(fmaxf(d[t][0], 0.f), fmaxf(d[t][1], 0.f));
+            h2[t][half * 2 + 1] = pack_bf16(fmaxf(d[t][2], 0.f), fmaxf(d[t][3], 0.f));
+        }
     }
 }
 
-// The output layer: y for rows g and g+8 in y0/y1 (valid on lanes with c == 0).
-__device__ __forceinline__ void mlp_output(const uint32_t (&h2)[4][4], const uint32_t* __restrict__ sfrag,
-                                           const float* __restrict__ sbias, float& y0, float& y1) {
+// The second hidden layer and the output layer, 16 hidden columns at a time (an
+// output product takes each as it is ready, in column order): y[t] for rows g
+// and g+8 of tile t, valid on lanes with c == 0.  With h2s the activations are
+// kept there.
+template <int T>
+__device__ __forceinline__ void mlp_rest(const uint32_t (&h)[T][4][4], const uint32_t* __restrict__ sfrag,
+                                         const float* __restrict__ sbias, float (&y)[T][2],
+                                         uint32_t (*h2s)[4][4] = nullptr) {
     const int lane = threadIdx.x & 31, c = lane & 3;
     const float b3 = (c == 0) ? sbias[128] : 0.f;
-    float d0 = b3, d1 = 0.f, d2 = b3, d3 = 0.f;
+    float d[T][4];
+#pragma unroll
+    for (int t = 0; t < T; ++t) { d[t][0] = d[t][2] = b3; d[t][1] = d[t][3] = 0.f; }
 #pragma unroll
     for (int kc = 0; kc < 4; ++kc) {
-        const uint32_t* bf = sfrag + F_W3 + kc * 64 + lane * 2;
-        mma_bf16(d0, d1, d2, d3, h2[kc][0], h2[kc][1], h2[kc][2], h2[kc][3], bf[0], bf[1]);
+        uint32_t h2[T][4];
+        mlp_layer2<T>(kc, h, sfrag, sbias, h2);
+        const uint2 w = *reinterpret_cast<const uint2*>(sfrag + F_W3 + kc * 64 + lane * 2);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            mma_bf16(d[t][0], d[t][1], d[t][2], d[t][3], h2[t][0], h2[t][1], h2[t][2], h2[t][3], w.x, w.y);
+            if (h2s) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) h2s[t][kc][e] = h2[t][e];
+            }
+        }
     }
-    y0 = d0;
-    y1 = d2;
-}
-
-// One warp's forward pass over a 16-row tile.
-__device__ __forceinline__ void mlp_tile(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         const uint32_t* __restrict__ sfrag, const float* __restrict__ sbias,
-                                         float& y0, float& y1) {
-    uint32_t h[4][4], h2[4][4];
-    mlp_hidden(a0, a1, a2, a3, sfrag, sbias, h, h2);
-    mlp_output(h2, sfrag, sbias, y0, y1);
+#pragma unroll
+    for (int t = 0; t < T; ++t) { y[t][0] = d[t][0]; y[t][1] = d[t][2]; }
 }
 
 __device__ __forceinline__ void load_net(const uint32_t* __restrict__ frag, const float* __restrict__ prm,
@@ -210,27 +292,102 @@ __device__ __forceinline__ void load_net(const uint32_t* __restrict__ frag, cons
     __syncthreads();
 }
 
-// Inference: y[i] for i < n, plus base[i] when base is given.
+// Inference on feature rows: y[i] for i < n.
 __global__ void __launch_bounds__(256) k_mlp_forward(const uint32_t* __restrict__ X, int n,
                                                      const uint32_t* __restrict__ frag,
-                                                     const float* __restrict__ prm, const float* __restrict__ base,
-                                                     float* __restrict__ y) {
-    __shared__ uint32_t sfrag[F_N];
-    __shared__ float sbias[132];
+                                                     const float* __restrict__ prm, float* __restrict__ y) {
+    __shared__ __align__(16) uint32_t sfrag[F_N];
+    __shared__ __align__(16) float sbias[132];
     load_net(frag, prm, sfrag, sbias);
     const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     const int warps = gridDim.x * (blockDim.x >> 5);
     for (int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile * 16 < n; tile += warps) {
         const int r0 = tile * 16 + g, r1 = r0 + 8;
-        uint32_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        if (r0 < n) { a0 = X[(size_t)r0 * 8 + c]; a2 = X[(size_t)r0 * 8 + c + 4]; }
-        if (r1 < n) { a1 = X[(size_t)r1 * 8 + c]; a3 = X[(size_t)r1 * 8 + c + 4]; }
-        float y0, y1;
-        mlp_tile(a0, a1, a2, a3, sfrag, sbias, y0, y1);
+        uint32_t a[1][4] = {{0, 0, 0, 0}}, h[1][4][4];
+        if (r0 < n) { a[0][0] = X[(size_t)r0 * 8 + c]; a[0][2] = X[(size_t)r0 * 8 + c + 4]; }
+        if (r1 < n) { a[0][1] = X[(size_t)r1 * 8 + c]; a[0][3] = X[(size_t)r1 * 8 + c + 4]; }
+        float yy[1][2];
+        mlp_layer1<1>(a, sfrag, sbias, h);
+        mlp_rest<1>(h, sfrag, sbias, yy);
         if (c == 0) {
-            if (r0 < n) y[r0] = base ? fadd(base[r0], y0) : y0;
-            if (r1 < n) y[r1] = base ? fadd(base[r1], y1) : y1;
+            if (r0 < n) y[r0] = yy[0][0];
+            if (r1 < n) y[r1] = yy[0][1];
         }
+    }
+}
+
+// Warm-start u = median indicator + network in one pass: each lane builds the
+// features of one cube, the warp runs its 32 cubes through the network as two
+// 16-row tiles that share every weight fragment read from shared memory, and
+// the outputs go back to the lane of their cube.
+//
+// Bytes: 16 + 4 NB read and 4 written per cube; the features (32 B), the median
+// (4 B) and the leaf number (4 B), which three kernels passed through memory
+// before, stay in registers.  Bound by the warp-level mma rate (44 mma per 16
+// cubes; about 236 TFLOP/s of mma.sync here, the rate that the backward pass
+// reaches too).  2.2 M cubes of 10 bins in 128 chunks: 68 + 44 + 83 us in three
+// kernels (a call 202 us) -> 104 us.
+//
+// The cube's chunk: SORTED = the boxes' index ranges ascend without overlap,
+// and the warp finds the last one that starts at or before its first cube by
+// bisection (128 chunks: 7 steps in place of a scan over all of them), each lane
+// stepping on from there.  Otherwise leaf_id names the chunk (the first in the
+// caller's order that holds the cube).
+constexpr int WS_WARPS = 8, WS_BLOCKS = 2;  // blocks per SM (2, 3 and 4 measure the same: 105, 104, 104 us)
+template <int NB, bool SORTED>
+__global__ void __launch_bounds__(WS_WARPS * 32, WS_BLOCKS)
+k_warm_start(int n, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
+             const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id,
+             const uint32_t* __restrict__ frag, const float* __restrict__ prm, float* __restrict__ u) {
+    __shared__ __align__(16) uint32_t sfrag[F_N];
+    __shared__ __align__(16) float sbias[132];
+    __shared__ FeatureTables tab;
+    __shared__ __align__(16) uint32_t sx[WS_WARPS][32 * 12];  // 12 words a row: fragment reads meet 32 banks
+    feature_tables<NB>(tab);
+    load_net(frag, prm, sfrag, sbias);  // ends with a block barrier
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    const bool vec = bins_aligned<NB>(hists);
+    uint32_t* xs = sx[warp];
+    for (int64_t i0 = ((int64_t)blockIdx.x * WS_WARPS + warp) * 32; i0 < n; i0 += (int64_t)gridDim.x * WS_WARPS * 32) {
+        const int i = (int)i0 + lane;
+        float med = 0.f;
+        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (i < n) {
+            uint32_t b[NB];
+            load_bins<NB>(hists + (size_t)i * NB, vec, b);
+            const uint4 cb = __ldg(cubes + i);
+            LeafBox box{0, 0, 0, 0, 0, 1.0f / (float)(1u << 21)};
+            if (SORTED) {
+                int lo = 0, hi = nleaf;  // first box that starts after the warp's first cube
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (__ldg(&boxes[mid].first) <= (uint32_t)i0) lo = mid + 1; else hi = mid;
+                }
+                int s = lo - 1;
+                while (s + 1 < nleaf && __ldg(&boxes[s + 1].first) <= (uint32_t)i) ++s;
+                if (s >= 0 && (uint32_t)i <= __ldg(&boxes[s].last)) box = boxes[s];
+            } else if (leaf_id) {
+                const int l = __ldg(leaf_id + i);
+                if (l >= 0) box = boxes[l];
+            }
+            med = feature_row<NB>(b, cb, box, tab, w);
+        }
+        __syncwarp();
+        *reinterpret_cast<uint4*>(xs + lane * 12) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(xs + lane * 12 + 4) = make_uint4(w[4], w[5], w[6], w[7]);
+        __syncwarp();
+        uint32_t a[2][4], h[2][4][4];
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[t][e] = xs[(t * 16 + (e & 1) * 8 + g) * 12 + c + (e >> 1) * 4];
+        mlp_layer1<2>(a, sfrag, sbias, h);
+        float y[2][2];
+        mlp_rest<2>(h, sfrag, sbias, y);
+        const int src = (lane & 7) * 4;  // cube r of a tile: row g = r & 7, first or second half
+        const float y00 = __shfl_sync(0xffffffffu, y[0][0], src), y01 = __shfl_sync(0xffffffffu, y[0][1], src);
+        const float y10 = __shfl_sync(0xffffffffu, y[1][0], src), y11 = __shfl_sync(0xffffffffu, y[1][1], src);
+        if (i < n) u[i] = fadd(med, lane < 8 ? y00 : (lane < 16 ? y01 : (lane < 24 ? y10 : y11)));
     }
 }
 
@@ -334,25 +491,26 @@ k_mlp_grad(const uint32_t* __restrict__ X, const float* __restrict__ t, const in
     const int a_row = (lane & 7) + ((lane >> 4) & 1) * 8, a_col = ((lane >> 3) & 1) * 8, b_row = lane & 15;
     for (int64_t r0 = (int64_t)blockIdx.x * ROWS; r0 < m; r0 += (int64_t)gridDim.x * ROWS) {
         int rows[2];
-        uint32_t a[4] = {0, 0, 0, 0};
+        uint32_t a[1][4] = {{0, 0, 0, 0}};
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             const int64_t b = r0 + lr + 8 * rr;
             rows[rr] = b < m ? (idx ? idx[b] : (int)b) : -1;
             if (rows[rr] >= 0) {
-                a[rr] = X[(size_t)rows[rr] * 8 + c];
-                a[rr + 2] = X[(size_t)rows[rr] * 8 + c + 4];
+                a[0][rr] = X[(size_t)rows[rr] * 8 + c];
+                a[0][rr + 2] = X[(size_t)rows[rr] * 8 + c + 4];
             }
-            sx[(lr + 8 * rr) * (GXP / 2) + c] = a[rr];
-            sx[(lr + 8 * rr) * (GXP / 2) + c + 4] = a[rr + 2];
+            sx[(lr + 8 * rr) * (GXP / 2) + c] = a[0][rr];
+            sx[(lr + 8 * rr) * (GXP / 2) + c + 4] = a[0][rr + 2];
         }
-        uint32_t h1[4][4], h2[4][4];
-        mlp_hidden(a[0], a[1], a[2], a[3], sfrag, sbias, h1, h2);
-        float y0, y1, dy0 = 0.f, dy1 = 0.f;
-        mlp_output(h2, sfrag, sbias, y0, y1);
+        uint32_t ha1[1][4][4], ha2[1][4][4];
+        mlp_layer1<1>(a, sfrag, sbias, ha1);
+        uint32_t (&h1)[4][4] = ha1[0], (&h2)[4][4] = ha2[0];
+        float y[1][2], dy0 = 0.f, dy1 = 0.f;
+        mlp_rest<1>(ha1, sfrag, sbias, y, ha2);
         if (c == 0) {  // dy = 2 (y - t) / m
-            if (rows[0] >= 0) { const float e = y0 - t[rows[0]]; lsum += e * e; dy0 = 2.f * e * inv_m; }
-            if (rows[1] >= 0) { const float e = y1 - t[rows[1]]; lsum += e * e; dy1 = 2.f * e * inv_m; }
+            if (rows[0] >= 0) { const float e = y[0][0] - t[rows[0]]; lsum += e * e; dy0 = 2.f * e * inv_m; }
+            if (rows[1] >= 0) { const float e = y[0][1] - t[rows[1]]; lsum += e * e; dy1 = 2.f * e * inv_m; }
             dys += dy0 + dy1;
         }
         dy0 = __shfl_sync(0xffffffffu, dy0, lane & 28);
@@ -678,10 +836,10 @@ extern "C" int tgvg_mlp_features(tgvg_ctx* ctx, const tgvg_cube* cubes, const ui
     }
     if (nbins == 8)
         k_mlp_features<8><<<grid, 256, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h,
-                                                         nleaf > 0 ? d_id : nullptr, d_l, d_x, nullptr);
+                                                         nleaf > 0 ? d_id : nullptr, d_l, d_x);
     else
         k_mlp_features<10><<<grid, 256, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h,
-                                                          nleaf > 0 ? d_id : nullptr, d_l, d_x, nullptr);
+                                                          nleaf > 0 ? d_id : nullptr, d_l, d_x);
     TGVG_LAUNCHED(ctx);
     TGVG_CK(ctx, cudaMemcpyAsync(X, d_x, sizeof(uint32_t) * 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
     TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -698,40 +856,44 @@ extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, i
     TGVG_CK(ctx, cudaMemcpyAsync(d_x, X, sizeof(uint32_t) * 8 * n, cudaMemcpyHostToDevice, ctx->stream));
     const int tiles = (int)((n + 15) / 16);
     const unsigned grid = (unsigned)std::min((tiles + 7) / 8, ctx->sm_count * 8);
-    k_mlp_forward<<<grid, 256, 0, ctx->stream>>>(d_x, (int)n, m->d_frag, m->d_prm, nullptr, d_y);
+    k_mlp_forward<<<grid, 256, 0, ctx->stream>>>(d_x, (int)n, m->d_frag, m->d_prm, d_y);
     TGVG_LAUNCHED(ctx);
     TGVG_CK(ctx, cudaMemcpyAsync(y, d_y, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
     TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return TGVG_OK;
 }
 
-// Warm-start u on the device: features, forward pass, plus the median
-// indicator (u = median + network).  Device cubes / histograms / output, host
-// leaves.  Called with ctx->mu held.
+// Warm-start u on the device (u = median + network).  Device cubes / histograms
+// / output, host leaves.  Called with ctx->mu held.
 static int warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_c, const uint32_t* d_h, int64_t n,
                           int32_t nbins, const tgvg_leaf* leaves, int32_t nleaf, float* d_u) {
-    auto* d_x = (uint32_t*)ctx->buf(B_M_X, sizeof(uint32_t) * 8 * n);
-    auto* d_med = (float*)ctx->buf(B_M_T, sizeof(float) * n);
-    auto* d_l = (tgvg_leaf*)ctx->buf(B_M_LEAVES, sizeof(tgvg_leaf) * std::max(1, nleaf));
-    auto* d_id = (int*)ctx->buf(B_M_LEAFID, sizeof(int) * n);
-    if (!d_x || !d_med || !d_l || !d_id) return TGVG_ERR_NOMEM;
+    auto* d_b = (LeafBox*)ctx->buf(B_M_BOXES, sizeof(LeafBox) * std::max(1, nleaf));
+    if (!d_b) return TGVG_ERR_NOMEM;
+    // Ranges that ascend without overlap (a treetop's) are found by bisection;
+    // any others keep the scan in the caller's order.
+    bool sorted = true;
+    std::vector<LeafBox> boxes(std::max(1, nleaf));
+    for (int l = 0; l < nleaf; ++l) {
+        boxes[l] = leaf_box(leaves[l]);
+        sorted = sorted && boxes[l].first <= boxes[l].last && (l == 0 || boxes[l].first > boxes[l - 1].last);
+    }
     if (nleaf > 0)
+        TGVG_CK(ctx, cudaMemcpyAsync(d_b, boxes.data(), sizeof(LeafBox) * nleaf, cudaMemcpyHostToDevice, ctx->stream));
+    int* d_id = nullptr;
+    if (!sorted) {
+        auto* d_l = (tgvg_leaf*)ctx->buf(B_M_LEAVES, sizeof(tgvg_leaf) * nleaf);
+        d_id = (int*)ctx->buf(B_M_LEAFID, sizeof(int) * n);
+        if (!d_l || !d_id) return TGVG_ERR_NOMEM;
         TGVG_CK(ctx, cudaMemcpyAsync(d_l, leaves, sizeof(tgvg_leaf) * nleaf, cudaMemcpyHostToDevice, ctx->stream));
-    const unsigned grid = (unsigned)((n + 255) / 256);
-    if (nleaf > 0) {
-        k_leaf_id<<<grid, 256, 0, ctx->stream>>>((int)n, nleaf, d_l, d_id);
+        k_leaf_id<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>((int)n, nleaf, d_l, d_id);
         TGVG_LAUNCHED(ctx);
     }
-    if (nbins == 8)
-        k_mlp_features<8><<<grid, 256, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h,
-                                                         nleaf > 0 ? d_id : nullptr, d_l, d_x, d_med);
-    else
-        k_mlp_features<10><<<grid, 256, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h,
-                                                          nleaf > 0 ? d_id : nullptr, d_l, d_x, d_med);
-    TGVG_LAUNCHED(ctx);
-    const int tiles = (int)((n + 15) / 16);
-    const unsigned fgrid = (unsigned)std::min((tiles + 7) / 8, ctx->sm_count * 8);
-    k_mlp_forward<<<fgrid, 256, 0, ctx->stream>>>(d_x, (int)n, m->d_frag, m->d_prm, d_med, d_u);
+    const unsigned grid = (unsigned)std::min<int64_t>((n + 32 * WS_WARPS - 1) / (32 * WS_WARPS), ctx->sm_count * WS_BLOCKS);
+    void (*k)(int, const uint4*, const uint32_t*, const LeafBox*, int, const int*, const uint32_t*, const float*, float*);
+    if (nbins == 8) k = sorted ? k_warm_start<8, true> : k_warm_start<8, false>;
+    else k = sorted ? k_warm_start<10, true> : k_warm_start<10, false>;
+    k<<<grid, WS_WARPS * 32, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h, d_b, nleaf, d_id,
+                                               m->d_frag, m->d_prm, d_u);
     TGVG_LAUNCHED(ctx);
     return TGVG_OK;
 }

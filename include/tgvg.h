@@ -182,13 +182,14 @@ int tgvg_set_timing(tgvg_ctx* ctx, int on);
  * (21) (in-memory and streaming semantics on levels whose dependencies all
  * point to earlier tiles once short runs of tiles are grouped, which holds for
  * Morton-sorted cubes; otherwise 14; never chosen by the autotuner), 22 = one
- * launch of a single 1024-thread block running every iteration, reading through
- * L1 (units of at most 4096 cubes), 23 = as 22 with the unit's state held in
- * shared memory for the whole launch (units of at most 2048 cubes; larger
- * units run 22), 24 = one thread-block cluster of 16 (else 8) CTAs whose
- * shared memories hold the unit's state, neighbours in other CTAs read through
- * distributed shared memory (units of at most 16 x 2816 cubes; larger units
- * run 14), -1 = let the online autotuner choose (default).  Results do not
+ * launch of a single 1024-thread block running every iteration, reading
+ * through L1 (units of at most 4096 cubes), 23 = one launch of one
+ * thread-block cluster of 1 to 8 CTAs running every iteration, one cube per
+ * thread with its state in registers and its neighbours' records in the
+ * cluster's shared memory (units of at most 2048 cubes; larger units run 22),
+ * 24 = the same on a cluster of 16 (else 8) CTAs (units of at most 16 x 1024
+ * cubes), above that the unit's state in the CTAs' shared memories (units of
+ * at most 16 x 2816 cubes; larger units run 14), -1 = let the online autotuner choose (default).  Results do not
  * depend on it. */
 int tgvg_set_schedule(tgvg_ctx* ctx, int32_t mode, int32_t cls, int32_t cfg);
 /* CUDA graphs for the level loop (1 = on, the default; 0 = off).  When every

@@ -191,8 +191,7 @@ struct tgvg_ctx {
     const void* fuse_cur = nullptr;    // the fused-schedule tables of the level being run (tgv.cu), or null
     const void* wave_cur = nullptr;    // the wavefront-schedule tables of the level being run (tgv.cu), or null
     int wave_occ[3][2] = {};           // blocks/SM of the wavefront kernel per mode [L2 loads, L1 loads]
-    bool smem_level_ready[3] = {};     // shared-memory limit of the tiny-level kernel raised, per mode
-    int smem_level_max = 0;            // dynamic shared memory that kernel may use (bytes)
+    int reg_max[3] = {-1, -1, -1};     // largest cluster of the register-resident level kernel per mode (-1 unknown)
     cudaEvent_t chk_ev[2] = {};        // stopping flags copied back while the next chunk of iterations runs
     int* chk_host = nullptr;           // pinned host copies of those flags (2 x chk_cap)
     int chk_cap = 0;

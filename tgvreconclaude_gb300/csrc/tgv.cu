@@ -367,7 +367,6 @@ struct IterArgs {
     int swap;             // per-launch schedules: dual sweep in reverse order, primal forward
     int band;             // per-launch schedules: warps stride over the whole unit (grid-stride band)
     int lend;             // end of the level's positions; cubes at lend and beyond are deeper
-    int gcap;             // single-block shared-memory schedule: room for staged out-of-unit values
     // per-launch sweep schedules (in-memory and streaming semantics): the unit's
     // -x/-y/-z neighbour table [3][n] with coarser neighbours replaced by
     // -2 - entry of gh, the compact copies of their gathered p/q values (or null)
@@ -1339,175 +1338,177 @@ __device__ __forceinline__ void dual_res(const DualLd& L, const float4& Po, cons
     res_terms<9>(w, o, dd, nd);
 }
 
-// ---- tiny levels in shared memory (schedule 23) -------------------------------
-// Every iteration of a unit of at most SMEM_MAX_N cubes in ONE launch of ONE
-// 1024-thread block that holds the unit's state, data term and neighbour
-// indices in shared memory (100 B per cube) for the whole launch: loaded once,
-// iterated with __syncthreads between the sweeps, written back once.  Cubes
-// outside the unit (coarser levels, the snapshot, other leaves) are read from
-// global memory; nothing writes them during the launch.  The arithmetic is the
-// split kernels' (dual_math, primal_math).
-constexpr int SMEM_MAX_N = 2048;
-static inline size_t smem_level_bytes(int n) { return size_t(n) * 100; }
-// Staged out-of-unit values follow the unit's arrays at a 16-byte boundary.
-static inline size_t smem_ghost_offset(int n) { return (smem_level_bytes(n) + 15) & ~size_t(15); }
+// ---- small levels in registers (schedules 23 and 24) --------------------------
+// Every iteration of a small unit in ONE launch of ONE thread-block cluster (1 to
+// 16 CTAs), one cube per thread.  A thread keeps its cube's u, v, bars, p, q and
+// data term in registers for the whole launch; shared memory holds only what
+// neighbours read: the bars, and per -x/-y/-z face the four p/q values that the
+// face's gather takes (as in the ghost tables), each one 16-byte record.  The
+// six neighbour records of a cube are six fixed shared-memory addresses in the
+// cluster's window, worked out once at launch, so an iteration has no index
+// arithmetic and no branch on where a neighbour lies:
+//   * in another CTA: that CTA's address (mapa);
+//   * outside the unit (coarser and deeper levels, other leaves, the snapshot),
+//     which does not change during the launch: a copy staged at launch;
+//   * missing: the cube's own bar (dual) or a zero record (primal).
+// Two barriers an iteration (the block's, or the cluster's hardware barrier with
+// release / acquire) order the sweeps; the last one also keeps every CTA's
+// shared memory alive until no other CTA reads it.  The arithmetic is the split
+// kernels' (dual_math, primal_math).
+//
+// Bound by latency: two dependent sweeps and two barriers.  us per iteration,
+// fixed count, best of the schedules that ran such a unit before (one block over
+// shared memory, cluster over L2, launches per sweep) -> this kernel: 22 cubes
+// 1.17 -> 0.46 (one CTA), 207: 1.23 -> 0.58, 485: 1.52 -> 1.11 (two CTAs),
+// 785: 2.18 -> 1.12, 1,895: 3.43 -> 1.08, 3,102: 3.33 -> 1.11 (16 CTAs),
+// 7,777: 3.88 -> 1.38, 12,002: 3.82 -> 1.65.
+constexpr int SMEM_MAX_N = 2048;    // schedule 23 takes units of at most this many cubes
+constexpr int REG_CTA_MAX = 1024;   // cubes (threads) per CTA
+// Schedule 23: cubes per CTA before another CTA is added.  A second CTA brings the
+// cluster barrier (0.6 us an iteration at one cube against 0.25), a full one the
+// issue slots of one SM; a 1,200-cube solve takes 847, 769 and 807 us at 128, 256 and 512.
+constexpr int REG_CTA_AIM = 256;
+// bars and three face records per cube, a zero record, at most six staged records per cube
+static inline size_t reg_level_bytes(int chunk) { return 16 * (10 * size_t(chunk) + 1); }
 
-template <int MODE>
-__device__ __forceinline__ float4 smem_bar(const IterArgs& a, const float4* s_bar, int j, const float4& own) {
-    if (j < 0) return own;
-    if (MODE != M_INMEM && (j & BORDER)) return a.snap[j & POS_MASK];
-    const unsigned li = (unsigned)(j - a.o);
-    return li < (unsigned)a.n ? s_bar[li] : a.bar[j];
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, unsigned rank) {
+    uint32_t out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+    return out;
+}
+template <bool ONE>
+__device__ __forceinline__ float4 ld_record(uint32_t addr) {
+    float4 r;
+    if (ONE)
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                     : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(addr) : "memory");
+    else
+        asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                     : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(addr) : "memory");
+    return r;
+}
+template <bool ONE>
+__device__ __forceinline__ void level_barrier() {
+    if (ONE) __syncthreads();
+    else cluster_barrier();
+}
+// What the -x / -y / -z gather (k = 0, 1, 2) takes of a cube's p and q.
+__device__ __forceinline__ float4 face_record(int k, const float4& A, const float4& B, float c5) {
+    return k == 0 ? make_float4(A.x, A.w, B.z, B.w)
+         : k == 1 ? make_float4(A.y, B.x, B.z, c5) : make_float4(A.z, B.y, B.w, c5);
 }
 
-template <int MODE>
-__device__ __forceinline__ bool smem_pq(const IterArgs& a, const float4* s_P, const float4* s_Q, const float* s_q5,
-                                        int jf, float4& A, float4& B, float& c5) {
-    if (jf < 0 || (MODE == M_STREAM && (jf & BORDER))) return false;
-    const int j = jf & POS_MASK;
-    const unsigned li = (unsigned)(j - a.o);
-    if (li < (unsigned)a.n) { A = s_P[li]; B = s_Q[li]; c5 = s_q5[li]; }
-    else { A = a.P4[j]; B = a.Q4[j]; c5 = a.Q1[j]; }
-    return true;
-}
-
-template <int MODE, bool STOP>
-__global__ void __launch_bounds__(CLUSTER_BLOCK) k_level_smem(IterArgs a) {
+// ONE: a single CTA (block barriers, plain shared-memory loads).
+template <int MODE, bool STOP, bool ONE>
+__global__ void __launch_bounds__(REG_CTA_MAX) k_level_reg(IterArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = a.n, o = a.o;
-    float4* s_uv = reinterpret_cast<float4*>(smem_raw);
-    float4* s_bar = s_uv + n;
-    float4* s_P = s_bar + n;
-    float4* s_Q = s_P + n;
-    float2* s_dat = reinterpret_cast<float2*>(s_Q + n);
-    float* s_q5 = reinterpret_cast<float*>(s_dat + n);
-    int* s_nb = reinterpret_cast<int*>(s_q5 + n);  // [6][n]
-    float4* s_gh = reinterpret_cast<float4*>(smem_raw + ((size_t(n) * 100 + 15) & ~size_t(15)));
     __shared__ int s_ng;
-    if (threadIdx.x == 0) s_ng = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int p = o + i;
-        s_uv[i] = a.uv[p]; s_bar[i] = a.bar[p]; s_P[i] = a.P4[p]; s_Q[i] = a.Q4[p];
-        s_dat[i] = a.dat[p]; s_q5[i] = a.Q1[p];
+    const int chunk = a.chunk, x = threadIdx.x, lane = x & 31;
+    const unsigned me = ONE ? 0u : cluster_rank();
+    float4* s_bar = reinterpret_cast<float4*>(smem_raw);
+    float4* s_face = s_bar + chunk;        // [3][chunk]
+    float4* s_zero = s_face + 3 * chunk;   // then the staged records
+    if (x == 0) { s_ng = 1; *s_zero = make_float4(0.f, 0.f, 0.f, 0.f); }
+    const int p = a.o + (int)me * chunk + x;
+    const bool mine = x < chunk && p < a.o + a.n;
+    DualLd L;
+    PrimalLd R;
+    uint32_t at[6] = {0, 0, 0, 0, 0, 0};
+    int slot = -1;
+    __syncthreads();
+    if (mine) {
+        R.U = a.uv[p]; R.D = a.dat[p];
+        L.b = a.bar[p]; L.P = a.P4[p]; L.Q = a.Q4[p]; L.q5 = a.Q1[p];
+        slot = MODE == M_STREAM ? __ldg(a.lid + p) : a.slot0;
+        s_bar[x] = L.b;
 #pragma unroll
-        for (int f = 0; f < 6; ++f) s_nb[f * n + i] = a.nb[(size_t)f * a.npos + p];
-    }
-    __syncthreads();
-    // Cubes outside the unit (coarser and deeper levels, other leaves, the
-    // snapshot) do not change during the launch: the values a face reads from
-    // one are staged once, so the iterations touch only shared memory.  A
-    // staged face holds slot -2 - g of s_gh: the neighbour's bars for the dual
-    // faces +x/+y/+z, the four gathered p/q values for the primal faces
-    // -x/-y/-z.  Faces beyond the room left in shared memory keep reading
-    // global memory.
-    for (int idx = threadIdx.x; idx < 6 * n; idx += blockDim.x) {
-        const int f = idx / n;
-        const int j = s_nb[idx];
-        if (j < 0) continue;
-        const bool border = MODE != M_INMEM && (j & BORDER);
-        const int jj = j & POS_MASK;
-        if (!border && (unsigned)(jj - o) < (unsigned)n) continue;  // inside the unit
-        if ((f & 1) && MODE == M_STREAM && border) continue;         // reads as zero already
-        float4 g;
-        if (!(f & 1)) {
-            g = border ? a.snap[jj] : a.bar[jj];
-        } else {
-            const float4 A = a.P4[jj], B = a.Q4[jj];
-            const float c5 = a.Q1[jj];
-            g = f == 1 ? make_float4(A.x, A.w, B.z, B.w)
-              : f == 3 ? make_float4(A.y, B.x, B.z, c5) : make_float4(A.z, B.y, B.w, c5);
+        for (int k = 0; k < 3; ++k) s_face[k * chunk + x] = face_record(k, L.P, L.Q, L.q5);
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_bar);
+        const uint32_t stage = (uint32_t)__cvta_generic_to_shared(s_zero);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            const int j = __ldg(a.nb + (size_t)f * a.npos + p), jj = j & POS_MASK, k = f >> 1;
+            const bool border = MODE != M_INMEM && j >= 0 && (j & BORDER);
+            uint32_t t;
+            if (f & 1 ? (j < 0 || (MODE == M_STREAM && border) || jj >= a.lend) : j < 0) {
+                t = f & 1 ? stage : base + 16u * x;
+                if (!ONE) t = cluster_addr(t, me);
+            } else if (!border && (unsigned)(jj - a.o) < (unsigned)a.n) {
+                const unsigned li = (unsigned)(jj - a.o), r = ONE ? 0u : li / (unsigned)chunk;
+                t = base + 16u * ((li - r * chunk) + (f & 1 ? (1 + k) * chunk : 0));
+                if (!ONE) t = cluster_addr(t, r);
+            } else {
+                const int g = atomicAdd(&s_ng, 1);  // at most six per cube: always room
+                s_zero[g] = f & 1 ? face_record(k, a.P4[jj], a.Q4[jj], a.Q1[jj]) : (border ? a.snap[jj] : a.bar[jj]);
+                t = stage + 16u * g;
+                if (!ONE) t = cluster_addr(t, me);
+            }
+            at[f] = t;
         }
-        const int slot = atomicAdd(&s_ng, 1);
-        if (slot < a.gcap) { s_gh[slot] = g; s_nb[idx] = -2 - slot; }
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (int k = 0; k < a.iters; ++k) {
-        const int it = a.it0 + k;
-        if (STOP && MODE != M_STREAM && *(volatile int*)(a.done + a.slot0)) break;
+    bool work = mine;
+    if (STOP && mine) work = __ldcg(a.done + slot) == 0;
+    level_barrier<ONE>();
+    // in-memory / OC semantics: one slot, met before this launch
+    const bool idle = STOP && MODE != M_STREAM && __ldcg(a.done + a.slot0) != 0;
+    for (int i = 0; i < a.iters && !idle; ++i) {
+        const int it = a.it0 + i;
         const bool res = STOP && ((it + 1) % a.check_every == 0 || it + 1 == a.iters_total);
-        WarpAcc wd, wp;
-        for (int i0 = 0; i0 < n; i0 += blockDim.x) {  // dual sweep (tgv.cpp:158-189)
-            const int i = i0 + (int)threadIdx.x;
-            bool work = i < n;
-            int slot = -1;
-            if (work) slot = (MODE == M_STREAM) ? __ldg(a.lid + o + i) : a.slot0;
-            if (STOP && work && MODE == M_STREAM) work = __ldcg(a.done + slot) == 0;
-            float dd = 0.f, nd = 0.f;
-            if (work) {
-                DualLd L;
-                L.b = s_bar[i]; L.P = s_P[i]; L.Q = s_Q[i]; L.q5 = s_q5[i];
-                const int j0 = s_nb[i], j2 = s_nb[2 * n + i], j4 = s_nb[4 * n + i];
-                L.B0 = j0 <= -2 ? s_gh[-2 - j0] : smem_bar<MODE>(a, s_bar, j0, L.b);
-                L.B2 = j2 <= -2 ? s_gh[-2 - j2] : smem_bar<MODE>(a, s_bar, j2, L.b);
-                L.B4 = j4 <= -2 ? s_gh[-2 - j4] : smem_bar<MODE>(a, s_bar, j4, L.b);
-                float4 Po, Qo;
-                float q5n;
-                dual_math(a, L, Po, Qo, q5n);
-                if (res) dual_res(L, Po, Qo, q5n, dd, nd);
-                s_P[i] = Po; s_Q[i] = Qo; s_q5[i] = q5n;
-            }
-            if (res) wd.add(work ? slot : -1, dd, nd, a.acc, 1, lane);
+        float dd = 0.f, nd = 0.f, dp = 0.f, np = 0.f;
+        if (work) {  // dual sweep (tgv.cpp:158-189)
+            L.B0 = ld_record<ONE>(at[0]);
+            L.B2 = ld_record<ONE>(at[2]);
+            L.B4 = ld_record<ONE>(at[4]);
+            float4 Po, Qo;
+            float q5n;
+            dual_math(a, L, Po, Qo, q5n);
+            if (STOP && res) dual_res(L, Po, Qo, q5n, dd, nd);
+            L.P = Po; L.Q = Qo; L.q5 = q5n;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s_face[k * chunk + x] = face_record(k, Po, Qo, q5n);
         }
-        if (res) wd.flush(a.acc, 1, lane);
-        __syncthreads();
-        for (int i0 = 0; i0 < n; i0 += blockDim.x) {  // primal sweep (tgv.cpp:191-230)
-            const int i = i0 + (int)threadIdx.x;
-            bool work = i < n;
-            int slot = -1;
-            if (work) slot = (MODE == M_STREAM) ? __ldg(a.lid + o + i) : a.slot0;
-            if (STOP && work && MODE == M_STREAM) work = __ldcg(a.done + slot) == 0;
-            float dd = 0.f, nd = 0.f;
-            if (work) {
-                PrimalLd L;
-                L.U = s_uv[i]; L.P = s_P[i]; L.Q = s_Q[i]; L.q5 = s_q5[i]; L.D = s_dat[i];
-                L.gp10 = L.gq10 = L.gq13 = L.gq14 = 0.f;
-                L.gp31 = L.gq31 = L.gq33 = L.gq35 = 0.f;
-                L.gp52 = L.gq52 = L.gq54 = L.gq55 = 0.f;
-                float4 A, B;
-                float c5;
-                const int j1 = s_nb[n + i], j3 = s_nb[3 * n + i], j5 = s_nb[5 * n + i];
-                if (j1 <= -2) {
-                    const float4 g = s_gh[-2 - j1];
-                    L.gp10 = g.x; L.gq10 = g.y; L.gq13 = g.z; L.gq14 = g.w;
-                } else if (smem_pq<MODE>(a, s_P, s_Q, s_q5, j1, A, B, c5)) {
-                    L.gp10 = A.x; L.gq10 = A.w; L.gq13 = B.z; L.gq14 = B.w;
-                }
-                if (j3 <= -2) {
-                    const float4 g = s_gh[-2 - j3];
-                    L.gp31 = g.x; L.gq31 = g.y; L.gq33 = g.z; L.gq35 = g.w;
-                } else if (smem_pq<MODE>(a, s_P, s_Q, s_q5, j3, A, B, c5)) {
-                    L.gp31 = A.y; L.gq31 = B.x; L.gq33 = B.z; L.gq35 = c5;
-                }
-                if (j5 <= -2) {
-                    const float4 g = s_gh[-2 - j5];
-                    L.gp52 = g.x; L.gq52 = g.y; L.gq54 = g.z; L.gq55 = g.w;
-                } else if (smem_pq<MODE>(a, s_P, s_Q, s_q5, j5, A, B, c5)) {
-                    L.gp52 = A.z; L.gq52 = B.y; L.gq54 = B.w; L.gq55 = c5;
-                }
-                float4 uvn, barn;
-                if (res) primal_math<true>(L, uvn, barn, dd, nd);
-                else primal_math<false>(L, uvn, barn, dd, nd);
-                s_uv[i] = uvn; s_bar[i] = barn;
-            }
-            if (res) wp.add(work ? slot : -1, dd, nd, a.acc, 0, lane);
+        level_barrier<ONE>();
+        if (work) {  // primal sweep (tgv.cpp:191-230)
+            const float4 g1 = ld_record<ONE>(at[1]), g3 = ld_record<ONE>(at[3]), g5 = ld_record<ONE>(at[5]);
+            R.P = L.P; R.Q = L.Q; R.q5 = L.q5;
+            R.gp10 = g1.x; R.gq10 = g1.y; R.gq13 = g1.z; R.gq14 = g1.w;
+            R.gp31 = g3.x; R.gq31 = g3.y; R.gq33 = g3.z; R.gq35 = g3.w;
+            R.gp52 = g5.x; R.gq52 = g5.y; R.gq54 = g5.z; R.gq55 = g5.w;
+            float4 uvn;
+            if (STOP && res) primal_math<true>(R, uvn, L.b, dp, np);
+            else primal_math<false>(R, uvn, L.b, dp, np);
+            R.U = uvn;
+            s_bar[x] = L.b;
         }
-        if (res) {
-            wp.flush(a.acc, 0, lane);
-            __syncthreads();
-            check_slots<MODE>(a, it);
+        if (STOP && res) {
+            WarpAcc w;
+            w.add(work ? slot : -1, dd, nd, a.acc, 1, lane);
+            w.flush(a.acc, 1, lane);
+            w.cur = -1;
+            w.add(work ? slot : -1, dp, np, a.acc, 0, lane);
+            w.flush(a.acc, 0, lane);
+            level_barrier<ONE>();
+            if (me == 0) check_slots<MODE>(a, it);
+            level_barrier<ONE>();
+            if (MODE != M_STREAM && __ldcg(a.done + a.slot0)) break;  // the same for every thread
+            if (work) work = __ldcg(a.done + slot) == 0;
+        } else {
+            level_barrier<ONE>();
         }
-        __syncthreads();
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int p = o + i;
-        a.uv[p] = s_uv[i]; a.bar[p] = s_bar[i]; a.P4[p] = s_P[i]; a.Q4[p] = s_Q[i]; a.Q1[p] = s_q5[i];
+    if (mine) {
+        a.uv[p] = R.U; a.bar[p] = L.b; a.P4[p] = L.P; a.Q4[p] = L.Q; a.Q1[p] = L.q5;
     }
 }
 
 // ---- small levels in distributed shared memory (schedule 24) -------------------
-// As k_level_smem for a unit of up to DSM_MAX_CHUNK cubes per CTA of one
-// thread-block cluster (8 or 16 CTAs of 1024 threads): each CTA holds the
+// Units beyond one cube per thread of a cluster: up to DSM_MAX_CHUNK cubes per
+// CTA of one thread-block cluster (8 or 16 CTAs of 1024 threads).  Each CTA holds the
 // state and data term of its contiguous chunk in its own shared memory (76 B
 // per cube; the neighbour indices stay in global memory), and a neighbour in
 // another CTA's chunk is read from that CTA's shared memory through the
@@ -1522,11 +1523,6 @@ struct DsmView {  // this CTA's arrays; a remote rank's through map_shared_rank
     float4* uv; float4* bar; float4* P; float4* Q; float2* dat; float* q5;
 };
 
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // Generic address of the same shared-memory location in CTA `rank` of the cluster.
 template <class T>
 __device__ __forceinline__ T* dsm_map(T* p, unsigned rank) {
@@ -2266,11 +2262,12 @@ static int iter_occupancy(tgvg_ctx* ctx) {
 //   (k_fused_tma).
 // cfg 22: every iteration in one launch of a single 1024-thread block
 //   (k_level_cta), reading through L1, for units of up to 4096 cubes.
-// cfg 23: as 22 with the unit's state, data term and neighbour indices held in
-//   shared memory for the whole launch (k_level_smem), units of up to 2048 cubes.
-// cfg 24: one thread-block cluster of 16 (else 8) CTAs whose shared memories
-//   hold the unit's state, neighbours in other CTAs read through distributed
-//   shared memory (k_level_dsm), units of up to 16 (8) x 2816 cubes.
+// cfg 23: one launch of one thread-block cluster of 1 to 8 CTAs, one cube per
+//   thread with its state in registers and its neighbours' records in the
+//   cluster's shared memory (k_level_reg), units of up to 2048 cubes.
+// cfg 24: the same on a cluster of 16 (else 8) CTAs, units of up to 16 (8) x 1024
+//   cubes; above, the unit's state in the CTAs' shared memories (k_level_dsm),
+//   units of up to 16 (8) x 2816 cubes.
 // cfg 20 / 21: one ordered-wavefront launch per iteration (k_wave): each
 //   block runs the dual then the primal step of a group of 512-cube tiles,
 //   after the tiles the primal step depends on have published their dual
@@ -2411,31 +2408,88 @@ static int effective_cfg(const tgvg_ctx* ctx, int cfg, int n) {
     const WaveSet* wz = static_cast<const WaveSet*>(ctx->wave_cur);
     if (fused_cfg(cfg) && (MODE == M_OC || !ctx->fuse_cur)) return CFG_BAND;
     if (wave_cfg(cfg) && (MODE == M_OC || !wz || !wz->ok)) return CFG_BAND;
-    if (cfg == CFG_SMEM && n > SMEM_MAX_N) return CFG_CTA;
-    if (cfg == CFG_DSM) {  // the cluster size is known once dsm_capacity ran (plan and tuning call it)
+    // (the cluster sizes are known once reg_capacity / dsm_capacity ran; plan and tuning call them)
+    if (cfg == CFG_SMEM && (n > SMEM_MAX_N || ctx->reg_max[MODE] == 0)) return CFG_CTA;
+    if (cfg == CFG_DSM && n > ctx->reg_max[MODE] * REG_CTA_MAX) {
         const int cs = ctx->dsm_max[MODE];
         if (cs >= 0 && (cs == 0 || n > cs * DSM_MAX_CHUNK)) return CFG_BAND;
     }
     return cfg;
 }
 
-// Shared-memory limit of the tiny-level kernel, raised once (before any capture).
+// The register kernel for a unit of n cubes on cs CTAs.
+struct RegLaunch {
+    void (*k)(IterArgs);
+    int cs, chunk, threads;
+};
 template <int MODE>
-static int smem_level_setup(tgvg_ctx* ctx) {
-    if (ctx->smem_level_ready[MODE]) return TGVG_OK;
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess)
-        return ctx->cuda_fail(cudaGetLastError(), "shared memory opt-in limit");
-    // the unit's arrays at the largest unit size, plus what is left for staged values
-    const int bytes = std::max((int)smem_ghost_offset(SMEM_MAX_N), optin - 1024);
-    ctx->smem_level_max = bytes;
-    cudaError_t e = cudaFuncSetAttribute((const void*)k_level_smem<MODE, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute((const void*)k_level_smem<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 bytes);
-    if (e != cudaSuccess) return ctx->cuda_fail(e, "shared memory limit");
-    ctx->smem_level_ready[MODE] = true;
+static RegLaunch reg_launch(int n, int cs, bool stop) {
+    RegLaunch r;
+    r.cs = cs;
+    r.chunk = (n + cs - 1) / cs;
+    r.threads = (r.chunk + 31) / 32 * 32;
+    if (cs == 1) r.k = stop ? k_level_reg<MODE, true, true> : k_level_reg<MODE, false, true>;
+    else r.k = stop ? k_level_reg<MODE, true, false> : k_level_reg<MODE, false, false>;
+    return r;
+}
+
+// CTAs of schedule 23: one per REG_CTA_AIM cubes, a power of two.
+static int reg_ctas(int n) {
+    int cs = 1;
+    while (cs < 8 && n > cs * REG_CTA_AIM) cs *= 2;
+    return cs;
+}
+
+static cudaError_t cluster_config(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int cs, int threads, size_t smem,
+                                  cudaStream_t st) {
+    lc = cudaLaunchConfig_t{};
+    lc.gridDim = dim3(cs);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaSuccess;
+}
+
+// Largest cluster of full-size CTAs the register kernel can use (16, else 8,
+// else 0), with its kernels' attributes set; cached in the context (before any
+// capture).
+template <int MODE>
+static int reg_capacity(tgvg_ctx* ctx, int* out) {
+    int& c = ctx->reg_max[MODE];
+    if (c < 0) {
+        c = 0;
+        const int bytes = (int)reg_level_bytes(REG_CTA_MAX);
+        bool ok = true;
+        for (int cs : {1, 2})
+            for (bool stop : {false, true}) {
+                const RegLaunch r = reg_launch<MODE>(cs, cs, stop);
+                ok = ok && cudaFuncSetAttribute((const void*)r.k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
+                               cudaSuccess;
+            }
+        for (int cs : {16, 8}) {
+            if (!ok) break;
+            bool fits = true;
+            for (bool stop : {false, true}) {
+                const RegLaunch r = reg_launch<MODE>(cs * REG_CTA_MAX, cs, stop);
+                if (cs == 16)
+                    fits = fits && cudaFuncSetAttribute((const void*)r.k,
+                                                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+                cudaLaunchConfig_t lc;
+                cudaLaunchAttribute at[1];
+                cluster_config(lc, at, cs, r.threads, reg_level_bytes(r.chunk), nullptr);
+                int nc = 0;
+                fits = fits && cudaOccupancyMaxActiveClusters(&nc, (const void*)r.k, &lc) == cudaSuccess && nc > 0;
+            }
+            if (fits) { c = cs; break; }
+            cudaGetLastError();
+        }
+        cudaGetLastError();
+    }
+    *out = c;
     return TGVG_OK;
 }
 
@@ -2619,6 +2673,27 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
         }
         return TGVG_OK;
     }
+    if (cfg == CFG_SMEM || cfg == CFG_DSM) {
+        int cs = 0;
+        const int rc = reg_capacity<MODE>(ctx, &cs);
+        if (rc) return rc;
+        const int use = cfg == CFG_SMEM ? reg_ctas(a.n) : cs;
+        if (cfg == CFG_SMEM && (cs == 0 || a.n > SMEM_MAX_N)) {
+            cfg = CFG_CTA;
+        } else if (a.n <= use * REG_CTA_MAX) {
+            const RegLaunch r = reg_launch<MODE>(a.n, use, stop);
+            a.chunk = r.chunk;
+            a.it0 = it0;
+            a.iters = count;
+            cudaLaunchConfig_t lc;
+            cudaLaunchAttribute at[1];
+            cluster_config(lc, at, r.cs, r.threads, reg_level_bytes(r.chunk), ctx->stream);
+            const cudaError_t e = cudaLaunchKernelEx(&lc, r.k, a);
+            if (e != cudaSuccess) return ctx->cuda_fail(e, "cluster launch");
+            ++ctx->kernels;
+            return TGVG_OK;
+        }
+    }
     if (cfg == CFG_DSM) {
         int cs = 0;
         const int rc = dsm_capacity<MODE>(ctx, &cs);
@@ -2645,20 +2720,6 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
             ++ctx->kernels;
             return TGVG_OK;
         }
-    }
-    if (cfg == CFG_SMEM && a.n > SMEM_MAX_N) cfg = CFG_CTA;
-    if (cfg == CFG_SMEM) {
-        const int rc = smem_level_setup<MODE>(ctx);
-        if (rc) return rc;
-        a.it0 = it0;
-        a.iters = count;
-        const size_t base = smem_ghost_offset(a.n);
-        const size_t sh = std::min((size_t)ctx->smem_level_max, base + size_t(16) * 6 * a.n);
-        a.gcap = (int)((sh - base) / 16);
-        if (stop) k_level_smem<MODE, true><<<1, CLUSTER_BLOCK, sh, ctx->stream>>>(a);
-        else k_level_smem<MODE, false><<<1, CLUSTER_BLOCK, sh, ctx->stream>>>(a);
-        TGVG_LAUNCHED(ctx);
-        return TGVG_OK;
     }
     if (cfg == CFG_CTA) {
         a.chunk = a.n;
@@ -2728,14 +2789,13 @@ static int tune_candidates(tgvg_ctx* ctx, int n, bool stop, std::vector<int>& ca
             last_grid = g;
         }
     if (n <= CTA_MAX_N) cands.push_back(CFG_CTA);
-    if (n <= SMEM_MAX_N) {
-        if ((rc = smem_level_setup<MODE>(ctx))) return rc;
-        cands.push_back(CFG_SMEM);
-    }
+    int rs = 0;
+    if ((rc = reg_capacity<MODE>(ctx, &rs))) return rc;
+    if (n <= SMEM_MAX_N && rs > 0) cands.push_back(CFG_SMEM);
     if (n <= 16 * DSM_MAX_CHUNK) {
         int cs = 0;
         if ((rc = dsm_capacity<MODE>(ctx, &cs))) return rc;
-        if (cs > 0 && n <= cs * DSM_MAX_CHUNK) cands.push_back(CFG_DSM);
+        if (n <= std::max(cs * DSM_MAX_CHUNK, rs * REG_CTA_MAX)) cands.push_back(CFG_DSM);
     }
     if (n <= CLUSTER_MAX_N) {
         int cs = 0;
@@ -2783,13 +2843,10 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
             int cs = 0;
             return cluster_capacity<MODE>(ctx, stop, &cs);
         }
-        if (tuned == CFG_SMEM) {
-            *cfg = effective_cfg<MODE>(ctx, tuned, n);
-            return smem_level_setup<MODE>(ctx);
-        }
-        if (tuned == CFG_DSM) {
+        if (tuned == CFG_SMEM || tuned == CFG_DSM) {
             int cs = 0;
-            rc = dsm_capacity<MODE>(ctx, &cs);
+            rc = reg_capacity<MODE>(ctx, &cs);
+            if (!rc && tuned == CFG_DSM) rc = dsm_capacity<MODE>(ctx, &cs);
             *cfg = effective_cfg<MODE>(ctx, tuned, n);
             return rc;
         }
@@ -2812,22 +2869,15 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
     // tolerance during the trials ends there without recording a pick).
     if ((int)cands.size() * TUNE_SEG * 2 <= iters) { *cfg = -1; return TGVG_OK; }
     // Untuned default (a tolerance-stopped solve, or too few iterations to
-    // tune), after the autotuner's picks on the benchmark octrees: the unit's
-    // state held on chip by one block (small units) or one cluster of 16 CTAs
-    // (mid-size units), else band order.  Each is a single launch for all of
-    // the unit's iterations or one launch per sweep, with no grid-wide barrier.
+    // tune), after the autotuner's picks on the benchmark octrees: one cube per
+    // thread of a cluster while the unit fits (a single launch for all of its
+    // iterations), else band order.
     *cfg = CFG_BAND;
-    if (n <= SMEM_MAX_N) {
-        if ((rc = smem_level_setup<MODE>(ctx))) return rc;
-        *cfg = effective_cfg<MODE>(ctx, CFG_SMEM, n);
-    } else if (n <= CTA_MAX_N) {
-        *cfg = CFG_CTA;
-    } else if (n <= 8192) {  // one cluster covers 16 SMs: beyond this per-sweep launches are faster
-        int cs = 0;
-        if ((rc = cluster_capacity<MODE>(ctx, stop, &cs))) return rc;
-        if (cs >= 16) *cfg = CFG_CLUSTER16;
-        else if (cs >= 8) *cfg = CFG_CLUSTER8;
-    }
+    int rs = 0;
+    if ((rc = reg_capacity<MODE>(ctx, &rs))) return rc;
+    if (rs > 0 && n <= SMEM_MAX_N) *cfg = CFG_SMEM;
+    else if (n <= rs * REG_CTA_MAX) *cfg = CFG_DSM;
+    else if (n <= CTA_MAX_N) *cfg = CFG_CTA;
     return TGVG_OK;
 }
 
@@ -2869,8 +2919,9 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
         ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, a.n))] = best;
         cfg = best;
     }
-    if (cfg == CFG_DSM) {
+    if (cfg == CFG_SMEM || cfg == CFG_DSM) {
         int cs = 0;
+        if ((rc = reg_capacity<MODE>(ctx, &cs))) return rc;
         if ((rc = dsm_capacity<MODE>(ctx, &cs))) return rc;
     }
     *used = effective_cfg<MODE>(ctx, cfg, a.n);

@@ -203,6 +203,7 @@ extern "C" int tgvg_destroy(tgvg_ctx* ctx) {
         std::lock_guard<std::mutex> lk(ctx->mu);
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
+        tgvg_release_mesh(ctx);
         for (auto& b : ctx->bufs)
             if (b.p) cudaFree(b.p);
         for (auto& e : ctx->ev) cudaEventDestroy(e);

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -168,6 +169,14 @@ enum BufId {
     B_COUNT
 };
 
+// The mesh whose data is in a context's surface output buffers (surface.cu),
+// shared by the context and the mesh; mu orders reads, moves to the host and frees.
+struct tgvg_mesh_link {
+    std::mutex mu;
+    tgvg_mesh* held = nullptr;
+    cudaStream_t stream = nullptr;
+};
+
 struct tgvg_ctx {
     int device = 0;
     int sm_count = 0;
@@ -205,6 +214,7 @@ struct tgvg_ctx {
     bool capturing = false;            // the level loop is being captured
     size_t device_budget = 0;          // solve footprint above which the state lives in host memory (0: never)
     bool paged_now = false;            // the running solve's state lives in host memory (no TMA-staged schedule)
+    std::shared_ptr<tgvg_mesh_link> mesh_link;  // set by the first surface extraction
     tgvg_ctx() {
         for (auto& m : tune)
             for (int& c : m) c = -1;
@@ -220,6 +230,9 @@ struct tgvg_ctx {
     int fail(int rc, const std::string& what);
     int cuda_fail(cudaError_t e, const char* what);
 };
+
+// The mesh on the device moves to host memory and the link's stream goes (surface.cu).
+void tgvg_release_mesh(tgvg_ctx* ctx);
 
 // Device bytes of a solve of n cubes, in round figures: state and its second
 // set 136 B, keys, hash, neighbour and order tables about 150 B, inputs and

@@ -34,6 +34,7 @@ void* tgvg_ctx::buf(int id, size_t bytes) {
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
+        ws_drop();
         e = cudaMalloc(&b.p, bytes);
         want = bytes;
     }
@@ -58,6 +59,7 @@ void* tgvg_ctx::host_backed(int id, size_t bytes) {
         b.cap = 0;
     }
     b.managed = false;
+    ws_drop();  // a state beyond the device budget: leave the device's memory to its slices
     cudaError_t e = cudaMallocManaged(&b.p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -78,6 +80,62 @@ void* tgvg_ctx::host_backed(int id, size_t bytes) {
     b.cap = bytes;
     b.managed = true;
     return b.p;
+}
+
+void* tgvg_ctx::ws_get(size_t bytes) {
+    // sizes rounded up by at most an eighth, so that calls of similar sizes meet
+    size_t unit = 512;
+    while (unit * 16 <= bytes) unit *= 2;
+    bytes = (bytes + unit - 1) / unit * unit;
+    // the smallest idle block that holds it without wasting more than it uses
+    size_t best = ws_idle.size();
+    for (size_t k = 0; k < ws_idle.size(); ++k)
+        if (ws_idle[k].bytes >= bytes && ws_idle[k].bytes <= 2 * bytes + (size_t(1) << 20) &&
+            (best == ws_idle.size() || ws_idle[k].bytes < ws_idle[best].bytes))
+            best = k;
+    if (best < ws_idle.size()) {
+        const Block b = ws_idle[best];
+        ws_idle.erase(ws_idle.begin() + best);
+        ws_idle_bytes -= b.bytes;
+        ws_used.push_back(b);
+        return b.p;
+    }
+    Block b{nullptr, bytes};
+    cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ws_drop();
+        e = cudaMalloc(&b.p, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        last_error = "cudaMalloc of " + std::to_string(bytes) + " bytes failed";
+        return nullptr;
+    }
+    ws_used.push_back(b);
+    return b.p;
+}
+
+void tgvg_ctx::ws_put(void* p) {
+    for (size_t k = 0; k < ws_used.size(); ++k)
+        if (ws_used[k].p == p) {
+            const Block b = ws_used[k];
+            ws_used.erase(ws_used.begin() + k);
+            ws_idle.push_back(b);
+            ws_idle_bytes += b.bytes;
+            break;
+        }
+    while (ws_idle_bytes > WS_CACHE_MAX && !ws_idle.empty()) {  // the oldest go first
+        ws_idle_bytes -= ws_idle.front().bytes;
+        cudaFree(ws_idle.front().p);  // waits for its uses
+        ws_idle.erase(ws_idle.begin());
+    }
+}
+
+void tgvg_ctx::ws_drop() {
+    for (const Block& b : ws_idle) cudaFree(b.p);
+    ws_idle.clear();
+    ws_idle_bytes = 0;
 }
 
 int tgvg_ctx::fail(int rc, const std::string& what) {
@@ -204,6 +262,7 @@ extern "C" int tgvg_destroy(tgvg_ctx* ctx) {
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
         tgvg_release_mesh(ctx);
+        ctx->ws_drop();
         for (auto& b : ctx->bufs)
             if (b.p) cudaFree(b.p);
         for (auto& e : ctx->ev) cudaEventDestroy(e);

@@ -227,6 +227,15 @@ struct tgvg_ctx {
     // are prefetched to the device (the state of solves larger than the
     // device budget).  A buffer changes kind by being reallocated.
     void* host_backed(int id, size_t bytes);
+    // Scratch blocks of calls whose sizes vary (merge, balance): taken from and
+    // given back to a cache of at most WS_CACHE_MAX bytes, all used on `stream`.
+    static constexpr size_t WS_CACHE_MAX = size_t(8) << 30;
+    struct Block { void* p; size_t bytes; };
+    std::vector<Block> ws_idle, ws_used;
+    size_t ws_idle_bytes = 0;
+    void* ws_get(size_t bytes);
+    void ws_put(void* p);
+    void ws_drop();  // frees the idle blocks
     int fail(int rc, const std::string& what);
     int cuda_fail(cudaError_t e, const char* what);
 };
@@ -269,5 +278,6 @@ int pyramid_dims(int32_t w, int32_t h, int32_t* dims);
 // Exclusive scan of n ints on the context stream; *total receives the sum (synchronises).
 int scan_exclusive(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, int64_t* total);
 int64_t scan_sums_len(int64_t n);
+int scan_tile_sums(tgvg_ctx* ctx, int* sums, int nt);
 int scan_exclusive_async(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, int* sums);
 }  // namespace tgvg

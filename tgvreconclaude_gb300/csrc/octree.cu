@@ -2,12 +2,14 @@
 // reference's kway_merge, src/merge.cpp:7-97) and the 2:1 balance
 // (balance_octree, src/balance.cpp:60-150).
 //
-// Merge.  The inputs are concatenated in order and stably radix-sorted by code,
-// so equal codes keep input order (the reference's heap leaves the order of
-// equal codes from different inputs to std::priority_queue; the two agree
-// whenever no code occurs in more than one input).  Runs of consecutive equal
-// (code, depth) collapse into one cube whose r_c is the run's float sum in
-// order divided by its length (merge.cpp:64-88).
+// Merge.  The code-sorted inputs are merged pairwise, neighbours first, in
+// ceil(log2 k) stable passes, so equal codes keep input order (the reference's
+// heap leaves the order of equal codes from different inputs to
+// std::priority_queue; the two agree whenever no code occurs in more than one
+// input).  An input that is not sorted is found by the first pass; all inputs
+// are then concatenated in order and stably radix-sorted by code.  Runs of
+// consecutive equal (code, depth) collapse into one cube whose r_c is the run's
+// float sum in order divided by its length (merge.cpp:64-88).
 //
 // Balance.  The reference processes a FIFO of cells one at a time, and each
 // cell's decisions read the cell sets as the cells before it left them.  The
@@ -98,32 +100,241 @@ __global__ void k_merge_keys(int64_t n, const tgvg_cube* __restrict__ c, unsigne
     idx[i] = i;
 }
 
-__global__ void k_merge_starts(int64_t n, const tgvg_cube* __restrict__ c, const long long* __restrict__ sidx,
-                               int* __restrict__ start) {
+__global__ void k_merge_gather(int64_t n, const tgvg_cube* __restrict__ c, const long long* __restrict__ sidx,
+                               tgvg_cube* __restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int s = 1;
-    if (i > 0) {
-        const tgvg_cube a = c[sidx[i - 1]], b = c[sidx[i]];
-        s = !(a.hi == b.hi && a.lo == b.lo && a.depth == b.depth);
-    }
-    start[i] = s;
+    if (i < n) out[i] = c[sidx[i]];
 }
 
-// One thread per run: the reference's pending-cube accumulation (merge.cpp:64-88).
-__global__ void k_merge_runs(int64_t n, const tgvg_cube* __restrict__ c, const long long* __restrict__ sidx,
-                             const int* __restrict__ start, const int* __restrict__ pos, tgvg_cube* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !start[i]) return;
-    tgvg_cube p = c[sidx[i]];
-    float sum = p.r_c;
-    uint32_t cnt = 1;
-    for (int64_t j = i + 1; j < n && !start[j]; ++j) {
-        sum = fadd(sum, c[sidx[j]].r_c);
-        ++cnt;
+// One stable pairwise merge pass (merge path): run [a, b) with run [b, e) of
+// src into dst[a..e), for every pair of a pass in one launch.  A block makes
+// MERGE_TILE consecutive outputs of one pair: two warps find how many of them,
+// and of those before them, come from the first run (a 32-way search along the
+// tile's diagonal), both segments go to shared memory, each thread merges
+// MERGE_ITEMS of them from its own diagonal, and the tile is written in order.
+// Equal codes: the first run's come first.
+//
+// Bound by bytes: 16 read and 16 written per cube and pass, whole records, so
+// nothing is gathered afterwards; what it reaches, 3.1 TB/s, is set by the
+// shared-memory merge.  2,048 outputs a block keep five to six blocks on an SM
+// (37 KB each), which covers the searches' latency.  16 lists of 400,000 cubes:
+// four passes of 63-66 us where a radix sort of (code, index) pairs took 680 us
+// with its keys, and its indices were gathered by the two kernels after it.
+constexpr int MERGE_THREADS = 256, MERGE_ITEMS = 8, MERGE_TILE = MERGE_THREADS * MERGE_ITEMS;
+// a spare record after every eight: threads whose records lie eight apart meet different banks
+__device__ __forceinline__ int merge_at(int i) { return i + (i >> 3); }
+struct MergePair {
+    int a, b, e;  // the two runs
+    int tile;     // the pair's first tile in the pass
+};
+__device__ __forceinline__ unsigned long long code_of(const uint4& c) { return ((unsigned long long)c.x << 32) | c.y; }
+
+// How many of the first d outputs come from the first run (whole warp).
+__device__ __forceinline__ int merge_split(const uint4* __restrict__ A, int na, const uint4* __restrict__ B, int nb,
+                                           int d, int lane) {
+    int lo = max(0, d - nb), hi = min(d, na);
+    while (lo < hi) {
+        const int step = (hi - lo + 31) / 32;
+        const int x = lo + lane * step + step - 1;
+        const bool first = x < hi && code_of(__ldg(A + x)) <= code_of(__ldg(B + (d - 1 - x)));
+        const int t = __popc(__ballot_sync(0xffffffffu, first));
+        lo = min(hi, lo + t * step);
+        hi = min(hi, lo + step - 1);
     }
-    p.r_c = fdiv(sum, (float)cnt);
-    out[pos[i]] = p;
+    return lo;
+}
+
+// bad (first pass only): set when a run is not sorted by code.
+__global__ void __launch_bounds__(MERGE_THREADS) k_merge_pass(const uint4* __restrict__ src, uint4* __restrict__ dst,
+                                                            const MergePair* __restrict__ pairs, int npairs,
+                                                            int* __restrict__ bad) {
+    __shared__ uint4 s[MERGE_TILE + MERGE_TILE / 8];
+    __shared__ int s_cut[2];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int lo = 0, hi = npairs - 1;  // last pair that starts at or before this tile
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(&pairs[mid].tile) <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const MergePair pr = pairs[lo];
+    const uint4 *A = src + pr.a, *B = src + pr.b;
+    const int na = pr.b - pr.a, nb = pr.e - pr.b;
+    const int d0 = ((int)blockIdx.x - pr.tile) * MERGE_TILE, cnt = min(MERGE_TILE, na + nb - d0), d1 = d0 + cnt;
+    if (warp < 2) {
+        const int x = merge_split(A, na, B, nb, warp ? d1 : d0, lane);
+        if (lane == 0) s_cut[warp] = x;
+    }
+    __syncthreads();
+    const int a0 = s_cut[0], a1 = s_cut[1], b0 = d0 - a0, b1 = d1 - a1;
+    if (a1 < a0 || b1 < b0) {  // only where a run is not sorted; the output is not used
+        if (bad && t == 0) atomicOr(bad, 1);
+        return;
+    }
+    const int ca = a1 - a0, cb = b1 - b0;
+    bool off = false;
+    for (int i = t; i < cnt; i += MERGE_THREADS) {
+        const bool in_a = i < ca;
+        const uint4* p = in_a ? A + a0 + i : B + b0 + (i - ca);
+        const uint4 v = __ldg(p);
+        s[merge_at(i)] = v;
+        if (bad && (in_a ? a0 + i + 1 < na : b0 + (i - ca) + 1 < nb)) off |= code_of(v) > code_of(__ldg(p + 1));
+    }
+    if (bad && off) atomicOr(bad, 1);
+    __syncthreads();
+    // this thread's diagonal inside the tile
+    const int d = min(t * MERGE_ITEMS, cnt);
+    int x = max(0, d - cb);
+    for (int h = min(d, ca); x < h;) {
+        const int mid = (x + h) >> 1;
+        if (code_of(s[merge_at(mid)]) <= code_of(s[merge_at(ca + d - 1 - mid)])) x = mid + 1; else h = mid;
+    }
+    int y = d - x;
+    // the heads of both runs stay in registers; a taken one is replaced by the next record
+    // (reads past a run's end meet the other run or the spare record and are not used)
+    uint4 r[MERGE_ITEMS], ha = s[merge_at(min(x, MERGE_TILE - 1))], hb = s[merge_at(min(ca + y, MERGE_TILE - 1))];
+#pragma unroll
+    for (int k = 0; k < MERGE_ITEMS; ++k) {
+        if (d + k >= cnt) break;
+        const bool first = y >= cb || (x < ca && code_of(ha) <= code_of(hb));
+        r[k] = first ? ha : hb;
+        x += first;
+        y += !first;
+        const uint4 h = s[merge_at(min(first ? x : ca + y, MERGE_TILE - 1))];
+        if (first) ha = h; else hb = h;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < MERGE_ITEMS; ++k)
+        if (d + k < cnt) s[merge_at(d + k)] = r[k];
+    __syncthreads();
+    uint4* out = dst + pr.a + d0;
+    for (int i = t; i < cnt; i += MERGE_THREADS) out[i] = s[merge_at(i)];
+}
+
+__device__ __forceinline__ bool same_cell(const uint4& a, const uint4& b) {
+    return a.x == b.x && a.y == b.y && a.w == b.w;
+}
+
+// Runs of equal (code, depth): per tile their number ...
+constexpr int RUN_THREADS = 256, RUN_TILE = 2048;
+__global__ void __launch_bounds__(RUN_THREADS) k_run_count(int64_t n, const uint4* __restrict__ c, int* __restrict__ sums) {
+    __shared__ int ws[RUN_THREADS / 32];
+    const int64_t base = (int64_t)blockIdx.x * RUN_TILE;
+    int cnt = 0;
+    for (int k = threadIdx.x; k < RUN_TILE; k += RUN_THREADS) {
+        const int64_t i = base + k;
+        if (i < n) cnt += i == 0 || !same_cell(__ldg(c + i), __ldg(c + i - 1));
+    }
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = cnt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int s = 0;
+        for (int w = 0; w < RUN_THREADS / 32; ++w) s += ws[w];
+        sums[blockIdx.x] = s;
+    }
+}
+
+// ... and, after a scan of those numbers, one cube per run: the reference's
+// pending-cube accumulation (merge.cpp:64-88).  A run's sum is a serial chain by
+// definition.  One thread takes a short run out of the tile in shared memory; a
+// run of RUN_SHORT cubes or more
+// (a coarse cell that thousands of pixels fall into) is left for a whole warp,
+// which loads 128 records ahead of the chain, so it advances at the latency of an
+// add and not of a load.  6.4 M cubes in 1.6 M runs: 325 us (a thread per run,
+// gathering) -> 99 us; with runs of more than 6 cubes left to warps 156 us.
+constexpr int RUN_SHORT = 41;  // 1 + a multiple of 4: four records are read at a time
+__global__ void __launch_bounds__(RUN_THREADS) k_run_emit(int64_t n, const uint4* __restrict__ c,
+                                                        const int* __restrict__ sums, uint4* __restrict__ out) {
+    __shared__ uint4 s[RUN_TILE + RUN_SHORT];  // the record before the tile, the tile, RUN_SHORT - 1 after it
+    __shared__ int ws[RUN_THREADS / 32];
+    __shared__ int s_long, s_off[RUN_TILE / RUN_SHORT + 1], s_out[RUN_TILE / RUN_SHORT + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * RUN_TILE;
+    int at = sums[blockIdx.x];
+    if (threadIdx.x == 0) s_long = 0;
+    for (int k = threadIdx.x; k < RUN_TILE + RUN_SHORT; k += RUN_THREADS) {
+        const int64_t i = base + k - 1;
+        if (i >= 0 && i < n) s[k] = __ldg(c + i);
+    }
+    __syncthreads();
+    for (int k0 = 0; k0 < RUN_TILE; k0 += RUN_THREADS) {
+        const int x = k0 + (int)threadIdx.x + 1;  // the record's place in s
+        const int64_t i = base + x - 1;
+        uint4 p = make_uint4(0, 0, 0, 0);
+        bool start = false;
+        if (i < n) {
+            p = s[x];
+            start = i == 0 || !same_cell(p, s[x - 1]);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, start);
+        if (lane == 0) ws[w] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int q = 0; q < RUN_THREADS / 32; ++q) {
+            if (q < w) before += ws[q];
+            all += ws[q];
+        }
+        if (start) {
+            const int o = at + before + __popc(m & ((1u << lane) - 1u));
+            float sum = __uint_as_float(p.z);
+            int cnt = 1;
+            bool more = true;
+            while (more && cnt < RUN_SHORT) {
+                uint4 v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = s[x + cnt + q];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    more = more && i + cnt < n && same_cell(v[q], p);
+                    if (more) { sum = fadd(sum, __uint_as_float(v[q].z)); ++cnt; }
+                }
+            }
+            // at RUN_SHORT the run may end here or go on: the warp's loop settles it
+            if (!more) {
+                out[o] = make_uint4(p.x, p.y, __float_as_uint(fdiv(sum, (float)cnt)), p.w);
+            } else {  // at least RUN_SHORT cubes: starts lie that far apart, so there is room
+                const int q = atomicAdd(&s_long, 1);
+                s_off[q] = x - 1;
+                s_out[q] = o;
+            }
+        }
+        at += all;
+        __syncthreads();
+    }
+    for (int q = w; q < s_long; q += RUN_THREADS / 32) {
+        const int64_t i = base + s_off[q];
+        const uint4 p = __ldg(c + i);
+        float sum = __uint_as_float(p.z);
+        uint32_t cnt = 1;
+        auto load = [&](int64_t j) {
+            return j < n ? __ldg(c + j) : make_uint4(~p.x, p.y, 0, p.w);  // past the end: another cell
+        };
+        uint4 v[4];
+        int64_t j = i + 1 + lane;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = load(j + 32 * e);
+        for (bool more = true; more; j += 128) {
+            uint4 nx[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) nx[e] = load(j + 128 + 32 * e);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const unsigned in = __ballot_sync(0xffffffffu, same_cell(v[e], p));
+                const int len = more ? (in == 0xffffffffu ? 32 : __ffs(~in) - 1) : 0;
+                if (len == 32) {
+#pragma unroll
+                    for (int r = 0; r < 32; ++r) sum = fadd(sum, __uint_as_float(__shfl_sync(0xffffffffu, v[e].z, r)));
+                } else {
+                    for (int r = 0; r < len; ++r) sum = fadd(sum, __uint_as_float(__shfl_sync(0xffffffffu, v[e].z, r)));
+                    more = false;
+                }
+                cnt += len;
+                v[e] = nx[e];
+            }
+        }
+        if (lane == 0) out[s_out[q]] = make_uint4(p.x, p.y, __float_as_uint(fdiv(sum, (float)cnt)), p.w);
+    }
 }
 
 // -------------------------------------------------------------- balance ---
@@ -319,23 +530,29 @@ uint64_t pow2_at_least(uint64_t x) {
     return c;
 }
 
-// Device memory of one balance run (owned here: the FIFO grows with its contents).
+// Device memory of one merge or balance run.  Blocks come from and go back to
+// the context's cache of such blocks (tgvg_ctx::ws_get / ws_put: at most
+// WS_CACHE_MAX bytes between calls, dropped when any allocation fails): a merge
+// made 9 and a balance about 30 cudaMalloc / cudaFree pairs per call, 0.9 ms of a
+// 2.8 ms merge and 4 ms of an 8.4 ms balance.  All uses of a block are on the
+// context's stream, so a block may be handed on while kernels still use it.
 struct Dev {
+    tgvg_ctx* ctx;
     std::vector<void*> ptrs;
+    explicit Dev(tgvg_ctx* c) : ctx(c) {}
     ~Dev() {
-        for (void* p : ptrs) cudaFree(p);
+        for (void* p : ptrs) ctx->ws_put(p);
     }
     template <class T>
     T* get(size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
+        void* p = ctx->ws_get(std::max<size_t>(count, 1) * sizeof(T));
+        if (p) ptrs.push_back(p);
         return (T*)p;
     }
     void release(void* p) {
         auto it = std::find(ptrs.begin(), ptrs.end(), p);
         if (it != ptrs.end()) {
-            cudaFree(p);
+            ctx->ws_put(p);
             ptrs.erase(it);
         }
     }
@@ -352,36 +569,100 @@ int merge_dev(tgvg_ctx* ctx, const tgvg_cube* const* in, const int64_t* counts, 
     if (n == 0) return TGVG_OK;
     if (n > (int64_t(1) << 31) - 1) return ctx->fail(TGVG_ERR_LIMIT, "more than 2^31 - 1 cubes");
     cudaStream_t st = ctx->stream;
-    Dev D;
+    Dev D(ctx);
     auto* cat = D.get<tgvg_cube>(n);
-    auto* key = D.get<unsigned long long>(n);
-    auto* skey = D.get<unsigned long long>(n);
-    auto* idx = D.get<long long>(n);
-    auto* sidx = D.get<long long>(n);
-    auto* start = D.get<int>(n);
-    auto* pos = D.get<int>(n);
-    if (!cat || !key || !skey || !idx || !sidx || !start || !pos) return ctx->fail(TGVG_ERR_NOMEM, "merge buffers");
-    int64_t off = 0;
-    for (int s = 0; s < k; ++s) {
-        if (counts[s])
-            TGVG_CK(ctx, cudaMemcpyAsync(cat + off, in[s], sizeof(tgvg_cube) * counts[s], cudaMemcpyHostToDevice, st));
-        off += counts[s];
-    }
-    k_merge_keys<<<grid_of(n, 256), 256, 0, st>>>(n, cat, key, idx);
-    TGVG_LAUNCHED(ctx);
-    size_t tb = 0;
-    TGVG_CK(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tb, key, skey, idx, sidx, (int)n, 0, 63, st));
-    void* tmp = D.get<char>(tb);
-    if (!tmp) return ctx->fail(TGVG_ERR_NOMEM, "merge sort buffer");
-    TGVG_CK(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, key, skey, idx, sidx, (int)n, 0, 63, st));
-    k_merge_starts<<<grid_of(n, 256), 256, 0, st>>>(n, cat, sidx, start);
-    TGVG_LAUNCHED(ctx);
-    int64_t runs = 0;
-    int rc = scan_exclusive(ctx, start, n, pos, &runs);
+    auto* oth = D.get<tgvg_cube>(n);
+    const int64_t ntiles = (n + RUN_TILE - 1) / RUN_TILE;
+    auto* sums = D.get<int>(ntiles + 2);  // [ntiles] total, [ntiles + 1] an input is not sorted
+    if (!cat || !oth || !sums) return ctx->fail(TGVG_ERR_NOMEM, "merge buffers");
+    auto upload = [&]() -> int {
+        int64_t off = 0;
+        for (int s = 0; s < k; ++s) {
+            if (counts[s])
+                TGVG_CK(ctx, cudaMemcpyAsync(cat + off, in[s], sizeof(tgvg_cube) * counts[s], cudaMemcpyHostToDevice, st));
+            off += counts[s];
+        }
+        return TGVG_OK;
+    };
+    int rc = upload();
     if (rc) return rc;
-    auto* res = D.get<tgvg_cube>(runs);
-    if (!res) return ctx->fail(TGVG_ERR_NOMEM, "merge output");
-    k_merge_runs<<<grid_of(n, 256), 256, 0, st>>>(n, cat, sidx, start, pos, res);
+    // The passes: runs of the concatenation, joined two by two until one is left
+    // (a single input still takes one pass, which checks that it is sorted).
+    std::vector<int> runs_at;  // run starts, then n
+    {
+        int64_t off = 0;
+        for (int s = 0; s < k; ++s) {
+            if (counts[s]) runs_at.push_back((int)off);
+            off += counts[s];
+        }
+        runs_at.push_back((int)n);
+    }
+    std::vector<MergePair> table;
+    struct Pass { int first, pairs, tiles; };
+    std::vector<Pass> passes;
+    do {
+        Pass ps{(int)table.size(), 0, 0};
+        std::vector<int> next;
+        for (size_t r = 0; r + 1 < runs_at.size(); r += 2) {
+            const int a = runs_at[r], b = runs_at[r + 1], e = r + 2 < runs_at.size() ? runs_at[r + 2] : b;
+            table.push_back({a, b, e, ps.tiles});
+            ps.tiles += (int)(((int64_t)e - a + MERGE_TILE - 1) / MERGE_TILE);
+            ++ps.pairs;
+            next.push_back(a);
+        }
+        next.push_back((int)n);
+        runs_at.swap(next);
+        passes.push_back(ps);
+    } while (runs_at.size() > 2);
+    auto* d_table = D.get<MergePair>(table.size());
+    if (!d_table) return ctx->fail(TGVG_ERR_NOMEM, "merge buffers");
+    TGVG_CK(ctx, cudaMemcpyAsync(d_table, table.data(), sizeof(MergePair) * table.size(), cudaMemcpyHostToDevice, st));
+    int* bad = sums + ntiles + 1;
+    TGVG_CK(ctx, cudaMemsetAsync(bad, 0, sizeof(int), st));
+    for (size_t q = 0; q < passes.size(); ++q) {
+        k_merge_pass<<<(unsigned)passes[q].tiles, MERGE_THREADS, 0, st>>>(
+            reinterpret_cast<const uint4*>(cat), reinterpret_cast<uint4*>(oth), d_table + passes[q].first,
+            passes[q].pairs, q == 0 ? bad : nullptr);
+        TGVG_LAUNCHED(ctx);
+        std::swap(cat, oth);
+    }
+    auto count_runs = [&](int64_t* total, bool* unsorted) -> int {
+        k_run_count<<<(unsigned)ntiles, RUN_THREADS, 0, st>>>(n, reinterpret_cast<const uint4*>(cat), sums);
+        TGVG_LAUNCHED(ctx);
+        const int src = scan_tile_sums(ctx, sums, (int)ntiles);
+        if (src) return src;
+        int h[2] = {0, 0};
+        TGVG_CK(ctx, cudaMemcpyAsync(h, sums + ntiles, sizeof(h), cudaMemcpyDeviceToHost, st));
+        TGVG_CK(ctx, cudaStreamSynchronize(st));
+        *total = h[0];
+        *unsorted = h[1] != 0;
+        return TGVG_OK;
+    };
+    int64_t runs = 0;
+    bool unsorted = false;
+    if ((rc = count_runs(&runs, &unsorted))) return rc;
+    if (unsorted) {  // stable radix sort of the concatenation
+        if ((rc = upload())) return rc;
+        auto* key = D.get<unsigned long long>(n);
+        auto* skey = D.get<unsigned long long>(n);
+        auto* idx = D.get<long long>(n);
+        auto* sidx = D.get<long long>(n);
+        if (!key || !skey || !idx || !sidx) return ctx->fail(TGVG_ERR_NOMEM, "merge buffers");
+        k_merge_keys<<<grid_of(n, 256), 256, 0, st>>>(n, cat, key, idx);
+        TGVG_LAUNCHED(ctx);
+        size_t tb = 0;
+        TGVG_CK(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tb, key, skey, idx, sidx, (int)n, 0, 63, st));
+        void* tmp = D.get<char>(tb);
+        if (!tmp) return ctx->fail(TGVG_ERR_NOMEM, "merge sort buffer");
+        TGVG_CK(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, key, skey, idx, sidx, (int)n, 0, 63, st));
+        k_merge_gather<<<grid_of(n, 256), 256, 0, st>>>(n, cat, sidx, oth);
+        TGVG_LAUNCHED(ctx);
+        std::swap(cat, oth);
+        if ((rc = count_runs(&runs, &unsorted))) return rc;
+    }
+    tgvg_cube* res = oth;  // at most n runs
+    k_run_emit<<<(unsigned)ntiles, RUN_THREADS, 0, st>>>(n, reinterpret_cast<const uint4*>(cat), sums,
+                                                        reinterpret_cast<uint4*>(res));
     TGVG_LAUNCHED(ctx);
     *count = runs;
     if (vec) {
@@ -413,7 +694,7 @@ int balance_dev(tgvg_ctx* ctx, const tgvg_cube* cubes, int64_t n, float r_root, 
     if (n == 0) return TGVG_OK;
     if (n > (int64_t(1) << 30)) return ctx->fail(TGVG_ERR_LIMIT, "more than 2^30 cubes");
     cudaStream_t st = ctx->stream;
-    Dev D;
+    Dev D(ctx);
     auto* c = D.get<tgvg_cube>(n);
     auto* bad = D.get<int>(1);
     unsigned long long* fc = D.get<unsigned long long>(1);

@@ -195,6 +195,13 @@ int scan_exclusive_async(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, 
     return TGVG_OK;
 }
 
+// In-place exclusive scan of nt numbers; sums[nt] receives the total.  Enqueued only.
+int scan_tile_sums(tgvg_ctx* ctx, int* sums, int nt) {
+    k_scan_sums<<<1, 1024, 0, ctx->stream>>>(sums, nt);
+    TGVG_LAUNCHED(ctx);
+    return TGVG_OK;
+}
+
 // out[i] = sum of in[0..i) for i < n; returns the total through *total (host).
 int scan_exclusive(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, int64_t* total) {
     *total = 0;

@@ -165,7 +165,7 @@ enum BufId {
     B_W_KEYS, B_W_SKEYS, B_W_KEEP, B_W_POS, B_W_UKEYS, B_W_DEP, B_W_DOFF, B_W_FLAG, B_W_CNT, B_W_TMP, B_W_TMP2,
     B_W_GSTART, B_LVENERGY,
     // coarser-neighbour ghost tables of the per-launch sweep schedules
-    B_G_PNB, B_G_VAL, B_G_MARK, B_G_IDS, B_G_SUMS, B_G_DNB, B_G_DVAL,
+    B_R_GX, B_R_PUB, B_G_PNB, B_G_VAL, B_G_MARK, B_G_IDS, B_G_SUMS, B_G_DNB, B_G_DVAL,
     B_COUNT
 };
 
@@ -204,7 +204,8 @@ struct tgvg_ctx {
     cudaEvent_t chk_ev[2] = {};        // stopping flags copied back while the next chunk of iterations runs
     int* chk_host = nullptr;           // pinned host copies of those flags (2 x chk_cap)
     int chk_cap = 0;
-    int dsm_max[3] = {-1, -1, -1};     // cluster size of the distributed-shared-memory kernel per mode (-1 unknown)
+    int grid_max[3] = {-1, -1, -1};    // blocks of the whole-GPU register kernel per mode (-1 unknown)
+    int grid_smem = 0;                 // dynamic shared memory of one of its blocks (bytes)
     cudaEvent_t lev_ev[2 * TGVG_MAX_LEVELS] = {};  // per-level start/end
     bool graphs = true;                // capture the level loop into a CUDA graph when possible
     std::vector<uint64_t> graph_key;   // problem signature of the cached graph

@@ -1506,145 +1506,210 @@ __global__ void __launch_bounds__(REG_CTA_MAX) k_level_reg(IterArgs a) {
     }
 }
 
-// ---- small levels in distributed shared memory (schedule 24) -------------------
-// Units beyond one cube per thread of a cluster: up to DSM_MAX_CHUNK cubes per
-// CTA of one thread-block cluster (8 or 16 CTAs of 1024 threads).  Each CTA holds the
-// state and data term of its contiguous chunk in its own shared memory (76 B
-// per cube; the neighbour indices stay in global memory), and a neighbour in
-// another CTA's chunk is read from that CTA's shared memory through the
-// cluster's distributed shared memory.  The hardware cluster barrier orders
-// the sweeps and makes each CTA's shared-memory writes visible to the others;
-// the last barrier of every iteration also keeps every CTA's shared memory
-// alive until no other CTA reads it.
-constexpr int DSM_MAX_CHUNK = 2816;
-static inline size_t dsm_level_bytes(int chunk) { return size_t(chunk) * 76; }
-
-struct DsmView {  // this CTA's arrays; a remote rank's through map_shared_rank
-    float4* uv; float4* bar; float4* P; float4* Q; float2* dat; float* q5;
+// ---- mid-size levels in registers over the whole GPU (schedule 24) -------------
+// Beyond a cluster's threads: one cooperative launch of one block per SM, K cubes
+// per thread, as k_level_reg, for all of the unit's iterations.  A block's
+// records are in its shared memory; what other blocks read of them (a cube's
+// bars, or one of its face records, only where some block asked for it at launch)
+// also goes to global memory (gx), and a neighbour in another block is read from
+// there through L2.  So of the 204 B that an iteration's two sweeps move per
+// cube, only the records at block borders still travel.
+//
+// The sweeps are separated by a barrier of the grid: a counter that only grows,
+// one addition and one polling thread per block.  (Each block's own word, polled
+// by all 152 threads of every block, took 8 us a barrier.)  The waits are bounded:
+// a block that gives up sets *err and ends, and so do the others when their own
+// waits run out.
+//
+// Bound by the two barriers and the L2 latency of each sweep's gathers.  us per
+// iteration, launches per sweep (schedule 14) -> this kernel: 31,728 cubes
+// 4.29 -> 3.69, 70,518: 4.54 -> 3.87, 128,846: 7.89 -> 4.38.  It takes the place
+// of a cluster holding up to 45,000 cubes in its shared memories (11.5 us at
+// 31,728).
+constexpr int GRID_K2_THREADS = 832;  // threads of a block at two cubes per thread (registers)
+struct GridArgs {
+    float4* gx;      // [4][n] bars and face records of cubes that other blocks read, then staged records
+    int* pub;        // [n] which of them: bit 0 bars, bit 1 + k face record k
+    unsigned* flag;  // the barrier's counter
+    int gcap;        // staged records with room in shared memory
 };
 
-// Generic address of the same shared-memory location in CTA `rank` of the cluster.
-template <class T>
-__device__ __forceinline__ T* dsm_map(T* p, unsigned rank) {
-    unsigned long long in = (unsigned long long)p, out;
-    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(in), "r"(rank));
-    return reinterpret_cast<T*>(out);
+__device__ __forceinline__ unsigned ld_acquire_u(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
 }
 
-template <int MODE>
-__device__ __forceinline__ float4 dsm_bar(const IterArgs& a, const DsmView& v, int chunk, unsigned me, int j,
-                                          const float4& own) {
-    if (j < 0) return own;
-    if (MODE != M_INMEM && (j & BORDER)) return a.snap[j & POS_MASK];
-    const unsigned li = (unsigned)(j - a.o);
-    if (li >= (unsigned)a.n) return a.bar[j];
-    const unsigned r = li / (unsigned)chunk, l = li - r * (unsigned)chunk;
-    return r == me ? v.bar[l] : dsm_map(v.bar, r)[l];
-}
-
-template <int MODE>
-__device__ __forceinline__ bool dsm_pq(const IterArgs& a, const DsmView& v, int chunk, unsigned me, int jf, float4& A,
-                                       float4& B, float& c5) {
-    if (jf < 0 || (MODE == M_STREAM && (jf & BORDER))) return false;
-    const int j = jf & POS_MASK;
-    const unsigned li = (unsigned)(j - a.o);
-    if (li >= (unsigned)a.n) { A = a.P4[j]; B = a.Q4[j]; c5 = a.Q1[j]; return true; }
-    const unsigned r = li / (unsigned)chunk, l = li - r * (unsigned)chunk;
-    if (r == me) { A = v.P[l]; B = v.Q[l]; c5 = v.q5[l]; }
-    else { A = dsm_map(v.P, r)[l]; B = dsm_map(v.Q, r)[l]; c5 = dsm_map(v.q5, r)[l]; }
-    return true;
-}
-
-template <int MODE, bool STOP>
-__global__ void __launch_bounds__(CLUSTER_BLOCK) k_level_dsm(IterArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int chunk = a.chunk;
-    const unsigned me = cluster_rank();
-    DsmView v;
-    v.uv = reinterpret_cast<float4*>(smem_raw);
-    v.bar = v.uv + chunk;
-    v.P = v.bar + chunk;
-    v.Q = v.P + chunk;
-    v.dat = reinterpret_cast<float2*>(v.Q + chunk);
-    v.q5 = reinterpret_cast<float*>(v.dat + chunk);
-    const int beg = a.o + (int)me * chunk, cnt = max(0, min(chunk, a.o + a.n - beg));
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const int p = beg + i;
-        v.uv[i] = a.uv[p]; v.bar[i] = a.bar[p]; v.P[i] = a.P4[p]; v.Q[i] = a.Q4[p];
-        v.dat[i] = a.dat[p]; v.q5[i] = a.Q1[p];
+// Barrier number `epoch` of the cooperative grid: thread 0 of each block adds one
+// to a counter that only grows and reads it until all blocks have.  False after
+// a wait that ran out (about a second).
+__device__ __forceinline__ bool flag_barrier(const GridArgs& g, unsigned epoch, int* err) {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.flag) : "memory");
+        const unsigned want = epoch * gridDim.x;
+        int spins = 0;
+        while ((int)(ld_acquire_u(g.flag) - want) < 0) {
+            if (++spins > (1 << 21)) {
+                atomicOr(err, 1);
+                ok = false;
+                break;
+            }
+        }
     }
-    cluster_barrier();
-    const int lane = threadIdx.x & 31;
-    for (int k = 0; k < a.iters; ++k) {
-        const int it = a.it0 + k;
-        if (STOP && MODE != M_STREAM && *(volatile int*)(a.done + a.slot0)) break;
+    return __syncthreads_and(ok) != 0;
+}
+
+// K = 1: neighbour places in registers; K > 1: in shared memory (registers are short).
+template <int MODE, bool STOP, int K>
+__global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_level_grid(IterArgs a, GridArgs g) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_ng;
+    const int T = blockDim.x, chunk = T * K, x = threadIdx.x, lane = x & 31;
+    const int beg = (int)blockIdx.x * chunk;
+    // [4 chunk] bars and face records, the zero record, [gcap] staged records, then the places (K > 1)
+    float4* s_rec = reinterpret_cast<float4*>(smem_raw);
+    float4* s_zero = s_rec + 4 * chunk;
+    int* s_at = reinterpret_cast<int*>(s_zero + 1 + g.gcap);
+    if (x == 0) { s_ng = 0; *s_zero = make_float4(0.f, 0.f, 0.f, 0.f); }
+    DualLd L[K];
+    float4 U[K];
+    int at[K == 1 ? 6 : 1];
+    int slot[K], pub[K];
+    bool mine[K], work[K];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int c = k * T + x, i = beg + c, p = a.o + i;
+        mine[k] = i < a.n;
+        slot[k] = -1;
+        if (!mine[k]) continue;
+        U[k] = a.uv[p];
+        L[k].b = a.bar[p]; L[k].P = a.P4[p]; L[k].Q = a.Q4[p]; L[k].q5 = a.Q1[p];
+        slot[k] = MODE == M_STREAM ? __ldg(a.lid + p) : a.slot0;
+        s_rec[c] = L[k].b;
+        g.gx[i] = L[k].b;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const float4 f = face_record(r, L[k].P, L[k].Q, L[k].q5);
+            s_rec[(1 + r) * chunk + c] = f;
+            g.gx[(size_t)(1 + r) * a.n + i] = f;
+        }
+        // a place >= 0 is a record in shared memory, < 0 the record ~place of gx
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            const int j = __ldg(a.nb + (size_t)f * a.npos + p), jj = j & POS_MASK, r = f >> 1;
+            const bool border = MODE != M_INMEM && j >= 0 && (j & BORDER);
+            int t;
+            if (f & 1 ? (j < 0 || (MODE == M_STREAM && border) || jj >= a.lend) : j < 0) {
+                t = f & 1 ? 4 * chunk : c;
+            } else if (!border && (unsigned)(jj - a.o) < (unsigned)a.n) {
+                const int li = jj - a.o, lc = li - beg, rec = f & 1 ? 1 + r : 0;
+                if ((unsigned)lc < (unsigned)chunk) {
+                    t = rec * chunk + lc;
+                } else {
+                    t = ~(rec * a.n + li);
+                    atomicOr(g.pub + li, 1 << rec);
+                }
+            } else {  // outside the unit: fixed during the launch
+                const float4 v = f & 1 ? face_record(r, a.P4[jj], a.Q4[jj], a.Q1[jj]) : (border ? a.snap[jj] : a.bar[jj]);
+                const int q = atomicAdd(&s_ng, 1);
+                if (q < g.gcap) {
+                    s_zero[1 + q] = v;
+                    t = 4 * chunk + 1 + q;
+                } else {
+                    const int e = 4 * a.n + f * a.n + i;
+                    g.gx[e] = v;
+                    t = ~e;
+                }
+            }
+            if (K == 1) at[f] = t;
+            else s_at[f * chunk + c] = t;
+        }
+    }
+    unsigned epoch = 0;
+    if (!flag_barrier(g, ++epoch, a.err)) return;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        pub[k] = mine[k] ? __ldcg(g.pub + beg + k * T + x) : 0;
+        work[k] = mine[k];
+        if (STOP && mine[k]) work[k] = __ldcg(a.done + slot[k]) == 0;
+    }
+    // in-memory / OC semantics: one slot, met before this launch (the same for every block)
+    const bool idle = STOP && MODE != M_STREAM && __ldcg(a.done + a.slot0) != 0;
+    auto rec = [&](int k, int f) {
+        const int t = K == 1 ? at[f] : s_at[f * chunk + k * T + x];
+        return t >= 0 ? s_rec[t] : __ldcg(g.gx + ~t);
+    };
+    for (int i = 0; i < a.iters && !idle; ++i) {
+        const int it = a.it0 + i;
         const bool res = STOP && ((it + 1) % a.check_every == 0 || it + 1 == a.iters_total);
         WarpAcc wd, wp;
-        for (int i0 = 0; i0 < cnt; i0 += blockDim.x) {  // dual sweep (tgv.cpp:158-189)
-            const int i = i0 + (int)threadIdx.x, p = beg + i;
-            bool work = i < cnt;
-            int slot = -1;
-            if (work) slot = (MODE == M_STREAM) ? __ldg(a.lid + p) : a.slot0;
-            if (STOP && work && MODE == M_STREAM) work = __ldcg(a.done + slot) == 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {  // dual sweep (tgv.cpp:158-189)
             float dd = 0.f, nd = 0.f;
-            if (work) {
-                DualLd L;
-                L.b = v.bar[i]; L.P = v.P[i]; L.Q = v.Q[i]; L.q5 = v.q5[i];
-                L.B0 = dsm_bar<MODE>(a, v, chunk, me, __ldg(a.nb + p), L.b);
-                L.B2 = dsm_bar<MODE>(a, v, chunk, me, __ldg(a.nb + 2 * a.npos + p), L.b);
-                L.B4 = dsm_bar<MODE>(a, v, chunk, me, __ldg(a.nb + 4 * a.npos + p), L.b);
+            const int c = k * T + x;
+            if (work[k]) {
+                L[k].B0 = rec(k, 0);
+                L[k].B2 = rec(k, 2);
+                L[k].B4 = rec(k, 4);
                 float4 Po, Qo;
                 float q5n;
-                dual_math(a, L, Po, Qo, q5n);
-                if (res) dual_res(L, Po, Qo, q5n, dd, nd);
-                v.P[i] = Po; v.Q[i] = Qo; v.q5[i] = q5n;
+                dual_math(a, L[k], Po, Qo, q5n);
+                if (STOP && res) dual_res(L[k], Po, Qo, q5n, dd, nd);
+                L[k].P = Po; L[k].Q = Qo; L[k].q5 = q5n;
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const float4 f = face_record(r, Po, Qo, q5n);
+                    s_rec[(1 + r) * chunk + c] = f;
+                    if (pub[k] & (2 << r)) __stcg(g.gx + (size_t)(1 + r) * a.n + beg + c, f);
+                }
             }
-            if (res) wd.add(work ? slot : -1, dd, nd, a.acc, 1, lane);
+            if (STOP && res) wd.add(work[k] ? slot[k] : -1, dd, nd, a.acc, 1, lane);
         }
-        if (res) wd.flush(a.acc, 1, lane);
-        cluster_barrier();
-        for (int i0 = 0; i0 < cnt; i0 += blockDim.x) {  // primal sweep (tgv.cpp:191-230)
-            const int i = i0 + (int)threadIdx.x, p = beg + i;
-            bool work = i < cnt;
-            int slot = -1;
-            if (work) slot = (MODE == M_STREAM) ? __ldg(a.lid + p) : a.slot0;
-            if (STOP && work && MODE == M_STREAM) work = __ldcg(a.done + slot) == 0;
+        if (STOP && res) wd.flush(a.acc, 1, lane);
+        if (!flag_barrier(g, ++epoch, a.err)) return;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {  // primal sweep (tgv.cpp:191-230)
             float dd = 0.f, nd = 0.f;
-            if (work) {
-                PrimalLd L;
-                L.U = v.uv[i]; L.P = v.P[i]; L.Q = v.Q[i]; L.q5 = v.q5[i]; L.D = v.dat[i];
-                L.gp10 = L.gq10 = L.gq13 = L.gq14 = 0.f;
-                L.gp31 = L.gq31 = L.gq33 = L.gq35 = 0.f;
-                L.gp52 = L.gq52 = L.gq54 = L.gq55 = 0.f;
-                float4 A, B;
-                float c5;
-                if (dsm_pq<MODE>(a, v, chunk, me, __ldg(a.nb + a.npos + p), A, B, c5)) {
-                    L.gp10 = A.x; L.gq10 = A.w; L.gq13 = B.z; L.gq14 = B.w;
-                }
-                if (dsm_pq<MODE>(a, v, chunk, me, __ldg(a.nb + 3 * a.npos + p), A, B, c5)) {
-                    L.gp31 = A.y; L.gq31 = B.x; L.gq33 = B.z; L.gq35 = c5;
-                }
-                if (dsm_pq<MODE>(a, v, chunk, me, __ldg(a.nb + 5 * a.npos + p), A, B, c5)) {
-                    L.gp52 = A.z; L.gq52 = B.y; L.gq54 = B.w; L.gq55 = c5;
-                }
-                float4 uvn, barn;
-                if (res) primal_math<true>(L, uvn, barn, dd, nd);
-                else primal_math<false>(L, uvn, barn, dd, nd);
-                v.uv[i] = uvn; v.bar[i] = barn;
+            const int c = k * T + x;
+            if (work[k]) {
+                const float4 g1 = rec(k, 1), g3 = rec(k, 3), g5 = rec(k, 5);
+                PrimalLd R;
+                R.U = U[k]; R.D = __ldg(a.dat + a.o + beg + c);
+                R.P = L[k].P; R.Q = L[k].Q; R.q5 = L[k].q5;
+                R.gp10 = g1.x; R.gq10 = g1.y; R.gq13 = g1.z; R.gq14 = g1.w;
+                R.gp31 = g3.x; R.gq31 = g3.y; R.gq33 = g3.z; R.gq35 = g3.w;
+                R.gp52 = g5.x; R.gq52 = g5.y; R.gq54 = g5.z; R.gq55 = g5.w;
+                float4 uvn;
+                if (STOP && res) primal_math<true>(R, uvn, L[k].b, dd, nd);
+                else primal_math<false>(R, uvn, L[k].b, dd, nd);
+                U[k] = uvn;
+                s_rec[c] = L[k].b;
+                if (pub[k] & 1) __stcg(g.gx + beg + c, L[k].b);
             }
-            if (res) wp.add(work ? slot : -1, dd, nd, a.acc, 0, lane);
+            if (STOP && res) wp.add(work[k] ? slot[k] : -1, dd, nd, a.acc, 0, lane);
         }
-        if (res) {
+        if (STOP && res) {
             wp.flush(a.acc, 0, lane);
-            cluster_barrier();
-            if (me == 0) check_slots<MODE>(a, it);
+            if (!flag_barrier(g, ++epoch, a.err)) return;
+            if (blockIdx.x == 0) check_slots<MODE>(a, it);
         }
-        cluster_barrier();
+        if (!flag_barrier(g, ++epoch, a.err)) return;
+        if (STOP && res) {
+            if (MODE != M_STREAM && __ldcg(a.done + a.slot0)) break;  // the same for every block
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (work[k]) work[k] = __ldcg(a.done + slot[k]) == 0;
+        }
     }
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const int p = beg + i;
-        a.uv[p] = v.uv[i]; a.bar[p] = v.bar[i]; a.P4[p] = v.P[i]; a.Q4[p] = v.Q[i]; a.Q1[p] = v.q5[i];
-    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (mine[k]) {
+            const int p = a.o + beg + k * T + x;
+            a.uv[p] = U[k]; a.bar[p] = L[k].b; a.P4[p] = L[k].P; a.Q4[p] = L[k].Q; a.Q1[p] = L[k].q5;
+        }
 }
 
 // The primal's neighbour p/q of faces 1/3/5 from their slots: shared memory
@@ -2266,8 +2331,8 @@ static int iter_occupancy(tgvg_ctx* ctx) {
 //   thread with its state in registers and its neighbours' records in the
 //   cluster's shared memory (k_level_reg), units of up to 2048 cubes.
 // cfg 24: the same on a cluster of 16 (else 8) CTAs, units of up to 16 (8) x 1024
-//   cubes; above, the unit's state in the CTAs' shared memories (k_level_dsm),
-//   units of up to 16 (8) x 2816 cubes.
+//   cubes; above, one cooperative launch of one block per SM with one or two
+//   cubes per thread (k_level_grid), units of up to 1664 cubes per SM.
 // cfg 20 / 21: one ordered-wavefront launch per iteration (k_wave): each
 //   block runs the dual then the primal step of a group of 512-cube tiles,
 //   after the tiles the primal step depends on have published their dual
@@ -2278,13 +2343,12 @@ static int iter_occupancy(tgvg_ctx* ctx) {
 //   tile hand-offs cost more than the traffic they save (largest three64
 //   level: 152 us per iteration against 119 us for schedule 14).
 static constexpr int TUNE_SEG = 16;
-static constexpr int N_PERSIST_CFG = 6;
 static constexpr int CFG_LEAN = 7;
 static constexpr int CFG_PF = 8, CFG_LEAN_PF = 9;
 static constexpr int CFG_SWAP = 12, CFG_SWAP_PF = 13, CFG_BAND = 14, CFG_BAND_SWAP = 15;
 static constexpr int CFG_BAND_ILP = 16, CFG_BAND_SWAP_ILP = 17, CFG_FUSED = 18, CFG_FUSED_TMA = 19;
-static constexpr int CFG_WAVE = 20, CFG_WAVE_L1 = 21, CFG_CTA = 22, CFG_SMEM = 23, CFG_DSM = 24;
-static constexpr int CTA_MAX_N = 4096;  // the single-block schedule is a candidate up to this unit size
+static constexpr int CFG_WAVE = 20, CFG_WAVE_L1 = 21, CFG_CTA = 22, CFG_SMEM = 23, CFG_REG = 24;
+static constexpr int CTA_MAX_N = 4096;  // where clusters cannot be used, one block takes units of up to this size
 static inline bool fused_cfg(int cfg) { return cfg == CFG_FUSED || cfg == CFG_FUSED_TMA; }
 static inline bool wave_cfg(int cfg) { return cfg == CFG_WAVE || cfg == CFG_WAVE_L1; }
 
@@ -2309,7 +2373,6 @@ static inline bool per_launch_cfg(int cfg) {
     return cfg == 0 || cfg == CFG_LEAN || cfg == CFG_PF || cfg == CFG_LEAN_PF || (cfg >= CFG_SWAP && cfg <= CFG_BAND_SWAP_ILP);
 }
 static constexpr int CFG_CLUSTER8 = 10, CFG_CLUSTER16 = 11;
-static constexpr int CLUSTER_MAX_N = 1 << 17;  // cluster schedules are candidates up to this unit size
 
 // Largest usable cluster size of k_level_cluster for this mode / stop variant
 // (16 when the device accepts non-portable clusters of 16 such CTAs, else 8, or
@@ -2400,6 +2463,19 @@ static int fused_occupancy(tgvg_ctx* ctx, bool tma, int* out) {
     return TGVG_OK;
 }
 
+// The whole-GPU register kernel for a unit of n cubes: cubes per thread (0: the
+// unit does not fit), threads and blocks.
+struct GridLaunch {
+    int k, threads, blocks;
+};
+static GridLaunch grid_launch(int n, int blocks) {
+    if (blocks <= 0) return {0, 0, 0};
+    const int per = (n + blocks - 1) / blocks;
+    const int k = per <= REG_CTA_MAX ? 1 : 2, t = ((per + k - 1) / k + 31) / 32 * 32;
+    if (k == 2 && t > GRID_K2_THREADS) return {0, 0, 0};
+    return {k, t, (n + k * t - 1) / (k * t)};
+}
+
 // The schedule a unit really runs: the fused and wavefront schedules need their
 // tables (in-memory and streaming semantics; for the wavefront, a level whose
 // dependencies all point backwards), else band order.
@@ -2408,12 +2484,9 @@ static int effective_cfg(const tgvg_ctx* ctx, int cfg, int n) {
     const WaveSet* wz = static_cast<const WaveSet*>(ctx->wave_cur);
     if (fused_cfg(cfg) && (MODE == M_OC || !ctx->fuse_cur)) return CFG_BAND;
     if (wave_cfg(cfg) && (MODE == M_OC || !wz || !wz->ok)) return CFG_BAND;
-    // (the cluster sizes are known once reg_capacity / dsm_capacity ran; plan and tuning call them)
+    // (the capacities are known once reg_capacity / grid_capacity ran; plan and tuning call them)
     if (cfg == CFG_SMEM && (n > SMEM_MAX_N || ctx->reg_max[MODE] == 0)) return CFG_CTA;
-    if (cfg == CFG_DSM && n > ctx->reg_max[MODE] * REG_CTA_MAX) {
-        const int cs = ctx->dsm_max[MODE];
-        if (cs >= 0 && (cs == 0 || n > cs * DSM_MAX_CHUNK)) return CFG_BAND;
-    }
+    if (cfg == CFG_REG && n > ctx->reg_max[MODE] * REG_CTA_MAX && grid_launch(n, ctx->grid_max[MODE]).k == 0) return CFG_BAND;
     return cfg;
 }
 
@@ -2493,49 +2566,46 @@ static int reg_capacity(tgvg_ctx* ctx, int* out) {
     return TGVG_OK;
 }
 
-// Cluster size of the distributed-shared-memory kernel (16 when the device
-// runs such clusters with the full shared-memory carve-out, else 8, else 0),
-// with the kernel's attributes set; cached in the context.
 template <int MODE>
-static int dsm_capacity(tgvg_ctx* ctx, int* out) {
-    int& c = ctx->dsm_max[MODE];
+static const void* grid_kernel(int k, bool stop) {
+    if (k == 1) return stop ? (const void*)k_level_grid<MODE, true, 1> : (const void*)k_level_grid<MODE, false, 1>;
+    return stop ? (const void*)k_level_grid<MODE, true, 2> : (const void*)k_level_grid<MODE, false, 2>;
+}
+// Fixed shared memory of a block: records, zero record, places; the rest is for staged records.
+static size_t grid_bytes(const GridLaunch& l) {
+    return 16 * (4 * (size_t)l.k * l.threads + 1) + (l.k > 1 ? 24 * (size_t)l.k * l.threads : 0);
+}
+
+// Blocks of the whole-GPU register kernel (one per SM; 0: unusable),
+// its kernels' attributes set and its scratch made; cached in the context
+// (before any capture).
+template <int MODE>
+static int grid_capacity(tgvg_ctx* ctx, int n, int* out) {
+    int& c = ctx->grid_max[MODE];
     if (c < 0) {
         c = 0;
-        const int bytes = (int)dsm_level_bytes(DSM_MAX_CHUNK);
-        const void* ks[2] = {(const void*)k_level_dsm<MODE, false>, (const void*)k_level_dsm<MODE, true>};
-        bool ok = true;
-        for (const void* k : ks)
-            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-        if (!ok) {
-            cudaGetLastError();
-        } else {
-            for (int cs : {16, 8}) {
-                bool allowed = true;
-                if (cs == 16)
-                    for (const void* k : ks)
-                        allowed = allowed &&
-                                  cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-                if (!allowed) { cudaGetLastError(); continue; }
-                bool fits = true;
-                for (const void* k : ks) {
-                    cudaLaunchConfig_t lc = {};
-                    lc.gridDim = dim3(cs);
-                    lc.blockDim = dim3(CLUSTER_BLOCK);
-                    lc.dynamicSmemBytes = (size_t)bytes;
-                    cudaLaunchAttribute at[1];
-                    at[0].id = cudaLaunchAttributeClusterDimension;
-                    at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                    lc.attrs = at;
-                    lc.numAttrs = 1;
-                    int nc = 0;
-                    fits = fits && cudaOccupancyMaxActiveClusters(&nc, k, &lc) == cudaSuccess && nc > 0;
-                }
-                if (fits) { c = cs; break; }
-                cudaGetLastError();
+        int optin = 0, coop = 0;
+        bool ok = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+                  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) == cudaSuccess && coop;
+        ctx->grid_smem = optin - 1024;
+        for (int k : {1, 2})
+            for (bool stop : {false, true}) {
+                int per = 0;
+                ok = ok &&
+                     cudaFuncSetAttribute(grid_kernel<MODE>(k, stop), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          ctx->grid_smem) == cudaSuccess &&
+                     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, grid_kernel<MODE>(k, stop),
+                                                                   k == 1 ? REG_CTA_MAX : GRID_K2_THREADS,
+                                                                   ctx->grid_smem) == cudaSuccess &&
+                     per > 0;
             }
-        }
+        if (ok) c = ctx->sm_count;
+        cudaGetLastError();
     }
     *out = c;
+    if (c > 0 && grid_launch(n, c).k > 0) {
+        if (!ctx->buf(B_R_GX, 160ull * n) || !ctx->buf(B_R_PUB, 4ull * (n + 1))) return TGVG_ERR_NOMEM;
+    }
     return TGVG_OK;
 }
 
@@ -2673,7 +2743,7 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
         }
         return TGVG_OK;
     }
-    if (cfg == CFG_SMEM || cfg == CFG_DSM) {
+    if (cfg == CFG_SMEM || cfg == CFG_REG) {
         int cs = 0;
         const int rc = reg_capacity<MODE>(ctx, &cs);
         if (rc) return rc;
@@ -2694,32 +2764,28 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
             return TGVG_OK;
         }
     }
-    if (cfg == CFG_DSM) {
-        int cs = 0;
-        const int rc = dsm_capacity<MODE>(ctx, &cs);
+    if (cfg == CFG_REG) {
+        int blocks = 0;
+        const int rc = grid_capacity<MODE>(ctx, a.n, &blocks);
         if (rc) return rc;
-        if (cs == 0 || a.n > cs * DSM_MAX_CHUNK) {
-            cfg = CFG_BAND;  // does not fit: band order
-        } else {
-            a.chunk = (a.n + cs - 1) / cs;
-            a.it0 = it0;
-            a.iters = count;
-            cudaLaunchConfig_t lc = {};
-            lc.gridDim = dim3(cs);
-            lc.blockDim = dim3(CLUSTER_BLOCK);
-            lc.dynamicSmemBytes = dsm_level_bytes(a.chunk);
-            lc.stream = ctx->stream;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-            lc.attrs = at;
-            lc.numAttrs = 1;
-            cudaError_t e = stop ? cudaLaunchKernelEx(&lc, k_level_dsm<MODE, true>, a)
-                                 : cudaLaunchKernelEx(&lc, k_level_dsm<MODE, false>, a);
-            if (e != cudaSuccess) return ctx->cuda_fail(e, "cluster launch");
-            ++ctx->kernels;
-            return TGVG_OK;
-        }
+        const GridLaunch l = grid_launch(a.n, blocks);
+        if (l.k == 0) return ctx->fail(TGVG_ERR_INVALID, "unit larger than the register schedule holds");
+        GridArgs g;
+        g.gx = (float4*)ctx->buf(B_R_GX, 160ull * a.n);
+        g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 1));
+        if (!g.gx || !g.pub) return TGVG_ERR_NOMEM;
+        g.flag = (unsigned*)(g.pub + a.n);
+        const size_t fixed = grid_bytes(l);
+        g.gcap = std::min(6 * l.k * l.threads, (int)((ctx->grid_smem - fixed) / 16));
+        a.it0 = it0;
+        a.iters = count;
+        TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 1), ctx->stream));
+        void* args[] = {&a, &g};
+        const cudaError_t e = cudaLaunchCooperativeKernel(grid_kernel<MODE>(l.k, stop), dim3(l.blocks), dim3(l.threads),
+                                                          args, fixed + 16 * (size_t)g.gcap, ctx->stream);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "cooperative launch");
+        ++ctx->kernels;
+        return TGVG_OK;
     }
     if (cfg == CFG_CTA) {
         a.chunk = a.n;
@@ -2773,36 +2839,28 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
     return TGVG_OK;
 }
 
-// Candidate schedules the autotuner times for a unit of n cubes: the two
-// per-iteration-launch variants and every persistent cfg whose grid differs.
+// Candidate schedules the autotuner times for a unit of n cubes.  A unit that
+// fits the registers of a cluster: those and band order (at 12,002 cubes 1.65 us
+// an iteration in registers, 3.8 and more with any other schedule).  Larger ones:
+// the variants with launches per iteration, and the whole GPU's registers while
+// the unit fits.  Not tried: one launch over software barriers and L2 (1-6), a
+// cluster over L2 (10, 11) and one block over L1 (22), which no size class picks
+// any more (2.2 us and up where registers take 0.3-1.1, 10.7 at 31,728 cubes
+// against 3.7).
 template <int MODE>
-static int tune_candidates(tgvg_ctx* ctx, int n, bool stop, std::vector<int>& cands) {
-    int cmax = 0, rc = coop_capacity<MODE>(ctx, stop, &cmax);
-    if (rc) return rc;
-    cands = {0, CFG_LEAN, CFG_PF, CFG_LEAN_PF, CFG_SWAP, CFG_SWAP_PF, CFG_BAND, CFG_BAND_SWAP, CFG_BAND_ILP,
-             CFG_BAND_SWAP_ILP};
-    int last_grid = -1;
-    if (n <= (1 << 22))
-        for (int k = 1; k <= N_PERSIST_CFG; ++k) {
-            const int g = persist_grid(n, k, cmax);
-            if (g != last_grid) cands.push_back(k);
-            last_grid = g;
-        }
-    if (n <= CTA_MAX_N) cands.push_back(CFG_CTA);
-    int rs = 0;
-    if ((rc = reg_capacity<MODE>(ctx, &rs))) return rc;
+static int tune_candidates(tgvg_ctx* ctx, int n, std::vector<int>& cands) {
+    int rc, rs = 0, gb = 0;
+    if ((rc = reg_capacity<MODE>(ctx, &rs)) || (rc = grid_capacity<MODE>(ctx, n, &gb))) return rc;
+    cands.clear();
     if (n <= SMEM_MAX_N && rs > 0) cands.push_back(CFG_SMEM);
-    if (n <= 16 * DSM_MAX_CHUNK) {
-        int cs = 0;
-        if ((rc = dsm_capacity<MODE>(ctx, &cs))) return rc;
-        if (n <= std::max(cs * DSM_MAX_CHUNK, rs * REG_CTA_MAX)) cands.push_back(CFG_DSM);
+    if (n <= rs * REG_CTA_MAX || grid_launch(n, gb).k > 0) cands.push_back(CFG_REG);
+    if (n <= rs * REG_CTA_MAX) {
+        cands.push_back(CFG_BAND);
+        return TGVG_OK;
     }
-    if (n <= CLUSTER_MAX_N) {
-        int cs = 0;
-        if ((rc = cluster_capacity<MODE>(ctx, stop, &cs))) return rc;
-        if (cs >= 8) cands.push_back(CFG_CLUSTER8);
-        if (cs >= 16) cands.push_back(CFG_CLUSTER16);
-    }
+    for (int c : {0, CFG_LEAN, CFG_PF, CFG_LEAN_PF, CFG_SWAP, CFG_SWAP_PF, CFG_BAND, CFG_BAND_SWAP, CFG_BAND_ILP,
+                  CFG_BAND_SWAP_ILP})
+        cands.push_back(c);
     if (MODE != M_OC && ctx->fuse_cur) {
         cands.push_back(CFG_FUSED);
         if (!ctx->paged_now) cands.push_back(CFG_FUSED_TMA);  // bulk copies stay on device-resident state
@@ -2810,11 +2868,16 @@ static int tune_candidates(tgvg_ctx* ctx, int n, bool stop, std::vector<int>& ca
     return TGVG_OK;
 }
 
+// Iterations of a candidate's trial.  A schedule that runs all iterations in one
+// launch loads its state and resolves its neighbours first (about 20 us over the
+// whole GPU): over 16 iterations that made 3.7 us look like 5.
+static int trial_iters(int cfg) { return cfg == CFG_SMEM || cfg == CFG_REG ? 4 * TUNE_SEG : TUNE_SEG; }
+
 // The schedule a unit of n cubes runs with, or -1 when the online autotuner
 // will first time the candidates on it.  The schedule for the unit's size
 // class (floor(log2 n)) is taken from the context's table; the first time a
 // class is met in a fixed-count solve with enough iterations, its first
-// segments try each candidate for TUNE_SEG iterations and keep the fastest
+// segments try each candidate (trial_iters) and keep the fastest per iteration
 // (the tried iterations count toward the solve).  Also makes sure the
 // occupancy figures the launches need are cached.
 template <int MODE>
@@ -2843,10 +2906,10 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
             int cs = 0;
             return cluster_capacity<MODE>(ctx, stop, &cs);
         }
-        if (tuned == CFG_SMEM || tuned == CFG_DSM) {
+        if (tuned == CFG_SMEM || tuned == CFG_REG) {
             int cs = 0;
             rc = reg_capacity<MODE>(ctx, &cs);
-            if (!rc && tuned == CFG_DSM) rc = dsm_capacity<MODE>(ctx, &cs);
+            if (!rc && tuned == CFG_REG) rc = grid_capacity<MODE>(ctx, n, &cs);
             *cfg = effective_cfg<MODE>(ctx, tuned, n);
             return rc;
         }
@@ -2863,20 +2926,22 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
         return TGVG_OK;
     }
     std::vector<int> cands;
-    if ((rc = tune_candidates<MODE>(ctx, n, stop, cands))) return rc;
+    if ((rc = tune_candidates<MODE>(ctx, n, cands))) return rc;
+    int trials = 0;
+    for (int c : cands) trials += trial_iters(c);
     // Tune when the trials are at most half the iterations: fixed-count solves,
     // and tolerance-stopped solves with a large cap (a unit that meets its
     // tolerance during the trials ends there without recording a pick).
-    if ((int)cands.size() * TUNE_SEG * 2 <= iters) { *cfg = -1; return TGVG_OK; }
+    if (trials * 2 <= iters) { *cfg = -1; return TGVG_OK; }
     // Untuned default (a tolerance-stopped solve, or too few iterations to
-    // tune), after the autotuner's picks on the benchmark octrees: one cube per
-    // thread of a cluster while the unit fits (a single launch for all of its
-    // iterations), else band order.
+    // tune), after the autotuner's picks on the benchmark octrees: the unit's
+    // state in registers, of a cluster or of the whole GPU, while it fits (a
+    // single launch for all of its iterations), else band order.
     *cfg = CFG_BAND;
-    int rs = 0;
-    if ((rc = reg_capacity<MODE>(ctx, &rs))) return rc;
+    int rs = 0, gb = 0;
+    if ((rc = reg_capacity<MODE>(ctx, &rs)) || (rc = grid_capacity<MODE>(ctx, n, &gb))) return rc;
     if (rs > 0 && n <= SMEM_MAX_N) *cfg = CFG_SMEM;
-    else if (n <= rs * REG_CTA_MAX) *cfg = CFG_DSM;
+    else if (n <= rs * REG_CTA_MAX || grid_launch(n, gb).k > 0) *cfg = CFG_REG;
     else if (n <= CTA_MAX_N) *cfg = CFG_CTA;
     return TGVG_OK;
 }
@@ -2887,17 +2952,18 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
     int it = 0, rc;
     if (cfg < 0) {
         std::vector<int> cands;
-        if ((rc = tune_candidates<MODE>(ctx, a.n, stop, cands))) return rc;
+        if ((rc = tune_candidates<MODE>(ctx, a.n, cands))) return rc;
         float best_ms = 1e30f;
         int best = 0;
         const int ns = unit_slots<MODE>(a.nslot);
         std::vector<int> done_h(stop ? ns : 0);
         for (int c : cands) {
             TGVG_CK(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
-            if ((rc = run_segment<MODE>(ctx, a, c, it, TUNE_SEG, stop, false))) return rc;
+            const int seg = trial_iters(c);
+            if ((rc = run_segment<MODE>(ctx, a, c, it, seg, stop, false))) return rc;
             TGVG_CK(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
             TGVG_CK(ctx, cudaEventSynchronize(ctx->ev[3]));
-            it += TUNE_SEG;
+            it += seg;
             if (stop) {
                 // A unit that met its tolerance during the trials is finished.  Its
                 // last segment stopped early and is not compared; the class keeps the
@@ -2914,15 +2980,16 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
             }
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
+            ms /= (float)seg;
             if (ms < best_ms) { best_ms = ms; best = c; }
         }
         ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, a.n))] = best;
         cfg = best;
     }
-    if (cfg == CFG_SMEM || cfg == CFG_DSM) {
+    if (cfg == CFG_SMEM || cfg == CFG_REG) {
         int cs = 0;
         if ((rc = reg_capacity<MODE>(ctx, &cs))) return rc;
-        if ((rc = dsm_capacity<MODE>(ctx, &cs))) return rc;
+        if ((rc = grid_capacity<MODE>(ctx, a.n, &cs))) return rc;
     }
     *used = effective_cfg<MODE>(ctx, cfg, a.n);
     const int eff = *used;
@@ -3561,7 +3628,8 @@ int tgv_solve_dev(tgvg_ctx* ctx, const tgvg_cube* d_cubes, const uint32_t* d_his
                               fused_ok ? fz0.barB : nullptr, fused_ok ? fz0.P4B : nullptr,
                               fused_ok ? fz0.Q4B : nullptr, fused_ok ? fz0.Q1B : nullptr,
                               fused_ok ? fz0.slot : nullptr, fused_ok ? fz0.halo : nullptr,
-                              g_pnb, g_val, g_mark, g_ids, g_sums, g_dnb, g_dval};
+                              g_pnb, g_val, g_mark, g_ids, g_sums, g_dnb, g_dval,
+                              ctx->bufs[B_R_GX].p, ctx->bufs[B_R_PUB].p};
         for (const void* q : ptrs) key.push_back((uint64_t)(uintptr_t)q);
         for (const Level& lvl : levels) {
             key.push_back(((uint64_t)lvl.d << 32) | (uint32_t)lvl.o);

@@ -159,7 +159,7 @@ enum BufId {
     B_S_SLOT, B_S_VFLAG, B_S_VID, B_S_VERTS, B_S_FACES, B_S_TN, B_S_VCNT, B_S_VSTART, B_S_VCUR, B_S_VLIST,
     B_S_NRM,
     // Stage 1
-    B_P_DEP, B_P_KEY, B_P_RC, B_P_DPT, B_P_KEEP, B_P_POS, B_P_THR, B_P_CKEY, B_P_CIDX, B_P_SKEY, B_P_SIDX,
+    B_P_DEP, B_P_KEY, B_P_RC, B_P_DPT, B_P_POS, B_P_CKEY, B_P_CIDX, B_P_SKEY, B_P_SIDX,
     B_P_OUT, B_P_TMP,
     // ordered-wavefront schedule tables
     B_W_KEYS, B_W_SKEYS, B_W_KEEP, B_W_POS, B_W_UKEYS, B_W_DEP, B_W_DOFF, B_W_FLAG, B_W_CNT, B_W_TMP, B_W_TMP2,

@@ -58,3 +58,28 @@ def test_graph_replays_follow_a_moved_scratch(oracle_lib):
         oracle_lib.tgv_solve(big, hb, None, "inmem", 0.5, 0.5, 6)[0].tobytes()
     for _ in range(3):
         assert api.tgv_solve(small, hs, None, "inmem", prm)[0].tobytes() == ref
+
+
+@pytest.mark.parametrize("mode", ["inmem", "oc", "stream"])
+@pytest.mark.parametrize("tol", [0.0, 1e-3])
+@pytest.mark.parametrize("n", [SM * 1664 + 1, 300_000, 520_001, 700_001])
+def test_units_in_shared_memory(oracle_lib, n, mode, tol):
+    """Schedule 24 beyond the registers: in shared memory while the unit fits,
+    band order above, bit for bit the oracle's."""
+    rng = np.random.default_rng(n)
+    cubes = _level(rng, n)
+    h = S.random_histograms(rng, len(cubes))
+    lv = None if mode == "inmem" else S.split_leaves(len(cubes), 1 if mode == "oc" else 5, rng, cubes, aligned=True)
+    iters = 25 if tol else 8
+    ref, rst = oracle_lib.tgv_solve(cubes, h, lv, mode, 0.5, 0.5, iters, nthreads=8,
+                                    **(dict(tol=tol, check_every=5) if tol else {}))
+    ctx = api.context()
+    ctx.set_schedule(mode, -1, 24)
+    try:
+        out, st = api.tgv_solve(cubes, h, lv, mode, api.TGVParams(0.5, 0.5, iters, tol=tol, check_every=5))
+    finally:
+        ctx.set_schedule(mode, -1, -1)
+    assert set(st["schedule"]) == ({24} if n < 530_000 else {24, 14})
+    assert out.tobytes() == ref.tobytes()
+    if tol:
+        assert st["iters_run"] == [r["iters_run"] for r in rst]

@@ -205,7 +205,7 @@ struct tgvg_ctx {
     int* chk_host = nullptr;           // pinned host copies of those flags (2 x chk_cap)
     int chk_cap = 0;
     int grid_max[3] = {-1, -1, -1};    // blocks of the whole-GPU register kernel per mode (-1 unknown)
-    int grid_smem = 0;                 // dynamic shared memory of one of its blocks (bytes)
+    int grid_smem = 0, chip_smem = 0;  // dynamic shared memory of a block of it / of the shared-memory kernel (bytes)
     cudaEvent_t lev_ev[2 * TGVG_MAX_LEVELS] = {};  // per-level start/end
     bool graphs = true;                // capture the level loop into a CUDA graph when possible
     std::vector<uint64_t> graph_key;   // problem signature of the cached graph

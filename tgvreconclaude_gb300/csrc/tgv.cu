@@ -1543,14 +1543,14 @@ __device__ __forceinline__ unsigned ld_acquire_u(const unsigned* p) {
 // Barrier number `epoch` of the cooperative grid: thread 0 of each block adds one
 // to a counter that only grows and reads it until all blocks have.  False after
 // a wait that ran out (about a second).
-__device__ __forceinline__ bool flag_barrier(const GridArgs& g, unsigned epoch, int* err) {
+__device__ __forceinline__ bool flag_barrier(unsigned* flag, unsigned epoch, int* err) {
     __syncthreads();
     bool ok = true;
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.flag) : "memory");
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(flag) : "memory");
         const unsigned want = epoch * gridDim.x;
         int spins = 0;
-        while ((int)(ld_acquire_u(g.flag) - want) < 0) {
+        while ((int)(ld_acquire_u(flag) - want) < 0) {
             if (++spins > (1 << 21)) {
                 atomicOr(err, 1);
                 ok = false;
@@ -1629,7 +1629,7 @@ __global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_l
         }
     }
     unsigned epoch = 0;
-    if (!flag_barrier(g, ++epoch, a.err)) return;
+    if (!flag_barrier(g.flag, ++epoch, a.err)) return;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         pub[k] = mine[k] ? __ldcg(g.pub + beg + k * T + x) : 0;
@@ -1669,7 +1669,7 @@ __global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_l
             if (STOP && res) wd.add(work[k] ? slot[k] : -1, dd, nd, a.acc, 1, lane);
         }
         if (STOP && res) wd.flush(a.acc, 1, lane);
-        if (!flag_barrier(g, ++epoch, a.err)) return;
+        if (!flag_barrier(g.flag, ++epoch, a.err)) return;
 #pragma unroll
         for (int k = 0; k < K; ++k) {  // primal sweep (tgv.cpp:191-230)
             float dd = 0.f, nd = 0.f;
@@ -1693,10 +1693,10 @@ __global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_l
         }
         if (STOP && res) {
             wp.flush(a.acc, 0, lane);
-            if (!flag_barrier(g, ++epoch, a.err)) return;
+            if (!flag_barrier(g.flag, ++epoch, a.err)) return;
             if (blockIdx.x == 0) check_slots<MODE>(a, it);
         }
-        if (!flag_barrier(g, ++epoch, a.err)) return;
+        if (!flag_barrier(g.flag, ++epoch, a.err)) return;
         if (STOP && res) {
             if (MODE != M_STREAM && __ldcg(a.done + a.slot0)) break;  // the same for every block
 #pragma unroll
@@ -1710,6 +1710,177 @@ __global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_l
             const int p = a.o + beg + k * T + x;
             a.uv[p] = U[k]; a.bar[p] = L[k].b; a.P4[p] = L[k].P; a.Q4[p] = L[k].Q; a.Q1[p] = L[k].q5;
         }
+}
+
+// ---- levels up to half a million cubes on chip (schedule 24) --------------------
+// Units too large for registers, up to about 535,000 cubes: one cooperative
+// launch of two blocks per SM in which each block keeps the bars and face records
+// of its consecutive cubes (64 B each: bars, p and q once) in shared memory and
+// their u and v in registers.  Per iteration and cube 32 B come from global
+// memory (the data term and the neighbour indices) instead of 204.  Records are
+// also stored to global memory where another block reads them (settled at launch,
+// pub).  Between the sweeps the grid meets at flag_barrier, after which ordinary
+// loads see what other blocks stored (release / acquire on the counter, then the
+// block's barrier).  The arithmetic is the split kernels'.
+//
+// Bound by the shared-memory traffic of about 250 B per cube and iteration, the
+// gathers' latency and the two barriers.  513,813 cubes: 18.3 us an iteration
+// with launches per sweep -> 12.6 us (512 threads with four cubes each 14.1, one
+// block of 1,024 per SM 13.8).  (Streaming the rest of a larger level in
+// the same launch was no gain: with 228 KB of shared memory in use the sweeps'
+// gathers lose L1, 65 -> 103 us at 1.94 M cubes; with 164 KB 65.3, as without.)
+constexpr int CHIP_THREADS = 640, CHIP_BLOCKS = 2, CHIP_K = 3;  // per SM; cubes per thread
+struct ChipArgs {
+    int* pub;        // [n] bit 0: the bars are read by another block, bit 1: p and q are
+    unsigned* flag;  // the barrier's counter
+    int rc;          // cubes per block
+};
+
+// What the -x / -y / -z gather (k = 0, 1, 2) gets from neighbour entry j (as primal_load_gather).
+template <int MODE, int k>
+__device__ __forceinline__ float4 gather_face(const IterArgs& a, int j) {
+    if (j >= 0 && !(MODE == M_STREAM && (j & BORDER)) && (j & POS_MASK) < a.lend) {
+        const int jj = j & POS_MASK;
+        return face_record(k, a.P4[jj], a.Q4[jj], k > 0 ? a.Q1[jj] : 0.f);
+    }
+    return j <= -2 ? __ldg(a.gh + (-2 - j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+template <int MODE, bool STOP>
+__global__ void __launch_bounds__(CHIP_THREADS, CHIP_BLOCKS) k_level_chip(IterArgs a, ChipArgs g) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int T = CHIP_THREADS;
+    const int x = threadIdx.x, lane = x & 31, rc = g.rc;
+    const int beg = (int)blockIdx.x * rc, cnt = max(0, min(rc, a.n - beg));
+    float4* s_rec = reinterpret_cast<float4*>(smem_raw);  // [4][rc]: bars, face records
+    uint8_t* s_pub = reinterpret_cast<uint8_t*>(s_rec + 4 * rc);
+    float4 U[CHIP_K];
+#pragma unroll
+    for (int k = 0; k < CHIP_K; ++k) {
+        const int c = k * T + x, p = a.o + beg + c;
+        if (c >= cnt) continue;
+        const float4 P = a.P4[p], Q = a.Q4[p];
+        const float q5 = a.Q1[p];
+        U[k] = a.uv[p];
+        s_rec[c] = a.bar[p];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) s_rec[(1 + f) * rc + c] = face_record(f, P, Q, q5);
+        // which cubes of other blocks this one reads
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            const int j = __ldg(a.nb + (size_t)f * a.npos + p), lj = j - a.o;
+            if (j < 0 || (MODE != M_INMEM && (j & BORDER)) || (unsigned)lj >= (unsigned)a.n ||
+                (unsigned)(lj - beg) < (unsigned)cnt)
+                continue;
+            const int bit = f & 1 ? 2 : 1;
+            if (!(__ldcg(g.pub + lj) & bit)) atomicOr(g.pub + lj, bit);
+        }
+    }
+    unsigned epoch = 0;
+    if (!flag_barrier(g.flag, ++epoch, a.err)) return;
+    for (int c = x; c < cnt; c += T) s_pub[c] = (uint8_t)__ldcg(g.pub + beg + c);
+    __syncthreads();
+    bool chk = true;  // streaming semantics: some slot has stopped, so cubes look at their own
+    for (int i = 0; i < a.iters; ++i) {
+        const int it = a.it0 + i;
+        const bool res = STOP && ((it + 1) % a.check_every == 0 || it + 1 == a.iters_total);
+        if (STOP && (i == 0 || it % a.check_every == 0)) {  // the flags change at check iterations only
+            int any = 0, all = 1;
+            for (int s = a.slot0 + x; s < a.slot0 + unit_slots<MODE>(a.nslot); s += T) {
+                const int d = __ldcg(a.done + s);
+                any |= d == 1;
+                all &= d != 0;
+            }
+            chk = __syncthreads_or(any) != 0;
+            if (__syncthreads_and(all)) break;  // the same for every block
+        }
+        auto slot_of = [&](int p) { return MODE == M_STREAM ? __ldg(a.lid + p) : a.slot0; };
+        auto running = [&](int p) { return !(STOP && MODE == M_STREAM && chk) || __ldcg(a.done + slot_of(p)) == 0; };
+        WarpAcc wd, wp;
+#pragma unroll
+        for (int k = 0; k < CHIP_K; ++k) {  // dual sweep (tgv.cpp:158-189)
+            const int c = k * T + x, p = a.o + beg + c;
+            const bool work = c < cnt && running(p);
+            float dd = 0.f, nd = 0.f;
+            if (work) {
+                DualLd L;
+                L.b = s_rec[c];
+                const float4 f0 = s_rec[rc + c], f1 = s_rec[2 * rc + c], f2 = s_rec[3 * rc + c];
+                L.P = make_float4(f0.x, f1.x, f2.x, f0.y);
+                L.Q = make_float4(f1.y, f2.y, f0.z, f0.w);
+                L.q5 = f1.w;
+                const int* jb = a.dnb ? a.dnb + (p - a.o) : a.nb + p;
+                const int js = a.dnb ? a.n : 2 * a.npos;
+                const int j0 = __ldg(jb), j2 = __ldg(jb + js), j4 = __ldg(jb + 2 * js);
+                auto bars = [&](int j) {
+                    const unsigned l = (unsigned)(j - a.o - beg);
+                    return l < (unsigned)cnt ? s_rec[l] : fetch_bar<MODE, false>(j, L.b, a.bar, a.snap, a.dgh);
+                };
+                L.B0 = bars(j0);
+                L.B2 = bars(j2);
+                L.B4 = bars(j4);
+                float4 Po, Qo;
+                float q5n;
+                dual_math(a, L, Po, Qo, q5n);
+                if (STOP && res) dual_res(L, Po, Qo, q5n, dd, nd);
+#pragma unroll
+                for (int f = 0; f < 3; ++f) s_rec[(1 + f) * rc + c] = face_record(f, Po, Qo, q5n);
+                if (s_pub[c] & 2) { a.P4[p] = Po; a.Q4[p] = Qo; a.Q1[p] = q5n; }
+            }
+            if (STOP && res) wd.add(work ? slot_of(p) : -1, dd, nd, a.acc, 1, lane);
+        }
+        if (STOP && res) wd.flush(a.acc, 1, lane);
+        if (!flag_barrier(g.flag, ++epoch, a.err)) return;
+#pragma unroll
+        for (int k = 0; k < CHIP_K; ++k) {  // primal sweep (tgv.cpp:191-230)
+            const int c = k * T + x, p = a.o + beg + c;
+            const bool work = c < cnt && running(p);
+            float dd = 0.f, nd = 0.f;
+            if (work) {
+                PrimalLd R;
+                R.U = U[k];
+                R.D = __ldg(a.dat + p);
+                const int* jb = a.pnb ? a.pnb + (p - a.o) : a.nb + a.npos + p;
+                const int js = a.pnb ? a.n : 2 * a.npos;
+                const int j1 = __ldg(jb), j3 = __ldg(jb + js), j5 = __ldg(jb + 2 * js);
+                const unsigned l1 = (unsigned)(j1 - a.o - beg), l3 = (unsigned)(j3 - a.o - beg), l5 = (unsigned)(j5 - a.o - beg);
+                const float4 g1 = l1 < (unsigned)cnt ? s_rec[rc + l1] : gather_face<MODE, 0>(a, j1);
+                const float4 g3 = l3 < (unsigned)cnt ? s_rec[2 * rc + l3] : gather_face<MODE, 1>(a, j3);
+                const float4 g5 = l5 < (unsigned)cnt ? s_rec[3 * rc + l5] : gather_face<MODE, 2>(a, j5);
+                R.gp10 = g1.x; R.gq10 = g1.y; R.gq13 = g1.z; R.gq14 = g1.w;
+                R.gp31 = g3.x; R.gq31 = g3.y; R.gq33 = g3.z; R.gq35 = g3.w;
+                R.gp52 = g5.x; R.gq52 = g5.y; R.gq54 = g5.z; R.gq55 = g5.w;
+                const float4 f0 = s_rec[rc + c], f1 = s_rec[2 * rc + c], f2 = s_rec[3 * rc + c];
+                R.P = make_float4(f0.x, f1.x, f2.x, f0.y);
+                R.Q = make_float4(f1.y, f2.y, f0.z, f0.w);
+                R.q5 = f1.w;
+                float4 uvn, b;
+                if (STOP && res) primal_math<true>(R, uvn, b, dd, nd);
+                else primal_math<false>(R, uvn, b, dd, nd);
+                U[k] = uvn;
+                s_rec[c] = b;
+                if (s_pub[c] & 1) a.bar[p] = b;
+            }
+            if (STOP && res) wp.add(work ? slot_of(p) : -1, dd, nd, a.acc, 0, lane);
+        }
+        if (STOP && res) {
+            wp.flush(a.acc, 0, lane);
+            if (!flag_barrier(g.flag, ++epoch, a.err)) return;
+            if (blockIdx.x == 0) check_slots<MODE>(a, it);
+        }
+        if (!flag_barrier(g.flag, ++epoch, a.err)) return;
+    }
+#pragma unroll
+    for (int k = 0; k < CHIP_K; ++k) {
+        const int c = k * T + x, p = a.o + beg + c;
+        if (c >= cnt) continue;
+        const float4 f0 = s_rec[rc + c], f1 = s_rec[2 * rc + c], f2 = s_rec[3 * rc + c];
+        a.uv[p] = U[k];
+        a.bar[p] = s_rec[c];
+        a.P4[p] = make_float4(f0.x, f1.x, f2.x, f0.y);
+        a.Q4[p] = make_float4(f1.y, f2.y, f0.z, f0.w);
+        a.Q1[p] = f1.w;
+    }
 }
 
 // The primal's neighbour p/q of faces 1/3/5 from their slots: shared memory
@@ -2332,7 +2503,9 @@ static int iter_occupancy(tgvg_ctx* ctx) {
 //   cluster's shared memory (k_level_reg), units of up to 2048 cubes.
 // cfg 24: the same on a cluster of 16 (else 8) CTAs, units of up to 16 (8) x 1024
 //   cubes; above, one cooperative launch of one block per SM with one or two
-//   cubes per thread (k_level_grid), units of up to 1664 cubes per SM.
+//   cubes per thread (k_level_grid), units of up to 1664 cubes per SM; above,
+//   one of two blocks per SM with the state in shared memory and registers
+//   (k_level_chip), units of up to about 3560 cubes per SM.
 // cfg 20 / 21: one ordered-wavefront launch per iteration (k_wave): each
 //   block runs the dual then the primal step of a group of 512-cube tiles,
 //   after the tiles the primal step depends on have published their dual
@@ -2468,6 +2641,10 @@ static int fused_occupancy(tgvg_ctx* ctx, bool tma, int* out) {
 struct GridLaunch {
     int k, threads, blocks;
 };
+// Cubes the shared-memory kernel holds (blocks: the cooperative kernels' blocks, 0 where they cannot run).
+static int chip_max(const tgvg_ctx* ctx, int blocks) {
+    return blocks > 0 ? CHIP_BLOCKS * blocks * std::min(CHIP_K * CHIP_THREADS, ctx->chip_smem / 65) : 0;
+}
 static GridLaunch grid_launch(int n, int blocks) {
     if (blocks <= 0) return {0, 0, 0};
     const int per = (n + blocks - 1) / blocks;
@@ -2486,7 +2663,7 @@ static int effective_cfg(const tgvg_ctx* ctx, int cfg, int n) {
     if (wave_cfg(cfg) && (MODE == M_OC || !wz || !wz->ok)) return CFG_BAND;
     // (the capacities are known once reg_capacity / grid_capacity ran; plan and tuning call them)
     if (cfg == CFG_SMEM && (n > SMEM_MAX_N || ctx->reg_max[MODE] == 0)) return CFG_CTA;
-    if (cfg == CFG_REG && n > ctx->reg_max[MODE] * REG_CTA_MAX && grid_launch(n, ctx->grid_max[MODE]).k == 0) return CFG_BAND;
+    if (cfg == CFG_REG && n > ctx->reg_max[MODE] * REG_CTA_MAX && n > chip_max(ctx, ctx->grid_max[MODE])) return CFG_BAND;
     return cfg;
 }
 
@@ -2567,6 +2744,11 @@ static int reg_capacity(tgvg_ctx* ctx, int* out) {
 }
 
 template <int MODE>
+static const void* chip_kernel(bool stop) {
+    return stop ? (const void*)k_level_chip<MODE, true> : (const void*)k_level_chip<MODE, false>;
+}
+
+template <int MODE>
 static const void* grid_kernel(int k, bool stop) {
     if (k == 1) return stop ? (const void*)k_level_grid<MODE, true, 1> : (const void*)k_level_grid<MODE, false, 1>;
     return stop ? (const void*)k_level_grid<MODE, true, 2> : (const void*)k_level_grid<MODE, false, 2>;
@@ -2599,11 +2781,24 @@ static int grid_capacity(tgvg_ctx* ctx, int n, int* out) {
                                                                    ctx->grid_smem) == cudaSuccess &&
                      per > 0;
             }
+        // the shared-memory kernel: two blocks per SM, 1 KB of each for the system
+        ctx->chip_smem = (optin + 1024) / CHIP_BLOCKS - 1024;
+        for (bool stop : {false, true}) {
+            int per = 0;
+            ok = ok &&
+                 cudaFuncSetAttribute(chip_kernel<MODE>(stop), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      ctx->chip_smem) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, chip_kernel<MODE>(stop), CHIP_THREADS,
+                                                               ctx->chip_smem) == cudaSuccess &&
+                 per >= CHIP_BLOCKS;
+        }
         if (ok) c = ctx->sm_count;
         cudaGetLastError();
     }
     *out = c;
-    if (c > 0 && grid_launch(n, c).k > 0) {
+    if (c > 0 && n <= chip_max(ctx, c) && grid_launch(n, c).k == 0) {
+        if (!ctx->buf(B_R_PUB, 4ull * (n + 1))) return TGVG_ERR_NOMEM;
+    } else if (grid_launch(n, c).k > 0) {
         if (!ctx->buf(B_R_GX, 160ull * n) || !ctx->buf(B_R_PUB, 4ull * (n + 1))) return TGVG_ERR_NOMEM;
     }
     return TGVG_OK;
@@ -2769,7 +2964,25 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
         const int rc = grid_capacity<MODE>(ctx, a.n, &blocks);
         if (rc) return rc;
         const GridLaunch l = grid_launch(a.n, blocks);
-        if (l.k == 0) return ctx->fail(TGVG_ERR_INVALID, "unit larger than the register schedule holds");
+        if (l.k == 0) {
+            if (a.n > chip_max(ctx, blocks))
+                return ctx->fail(TGVG_ERR_INVALID, "unit larger than the on-chip schedule holds");
+            ChipArgs g;
+            const int grid = CHIP_BLOCKS * ctx->sm_count;
+            g.rc = (a.n + grid - 1) / grid;
+            g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 1));
+            if (!g.pub) return TGVG_ERR_NOMEM;
+            g.flag = (unsigned*)(g.pub + a.n);
+            a.it0 = it0;
+            a.iters = count;
+            TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 1), ctx->stream));
+            void* args[] = {&a, &g};
+            const cudaError_t e = cudaLaunchCooperativeKernel(chip_kernel<MODE>(stop), dim3(grid), dim3(CHIP_THREADS),
+                                                              args, ctx->chip_smem, ctx->stream);
+            if (e != cudaSuccess) return ctx->cuda_fail(e, "cooperative launch");
+            ++ctx->kernels;
+            return TGVG_OK;
+        }
         GridArgs g;
         g.gx = (float4*)ctx->buf(B_R_GX, 160ull * a.n);
         g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 1));
@@ -2853,7 +3066,7 @@ static int tune_candidates(tgvg_ctx* ctx, int n, std::vector<int>& cands) {
     if ((rc = reg_capacity<MODE>(ctx, &rs)) || (rc = grid_capacity<MODE>(ctx, n, &gb))) return rc;
     cands.clear();
     if (n <= SMEM_MAX_N && rs > 0) cands.push_back(CFG_SMEM);
-    if (n <= rs * REG_CTA_MAX || grid_launch(n, gb).k > 0) cands.push_back(CFG_REG);
+    if (n <= rs * REG_CTA_MAX || n <= chip_max(ctx, gb)) cands.push_back(CFG_REG);
     if (n <= rs * REG_CTA_MAX) {
         cands.push_back(CFG_BAND);
         return TGVG_OK;
@@ -2941,7 +3154,7 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
     int rs = 0, gb = 0;
     if ((rc = reg_capacity<MODE>(ctx, &rs)) || (rc = grid_capacity<MODE>(ctx, n, &gb))) return rc;
     if (rs > 0 && n <= SMEM_MAX_N) *cfg = CFG_SMEM;
-    else if (n <= rs * REG_CTA_MAX || grid_launch(n, gb).k > 0) *cfg = CFG_REG;
+    else if (n <= rs * REG_CTA_MAX || n <= chip_max(ctx, gb)) *cfg = CFG_REG;
     else if (n <= CTA_MAX_N) *cfg = CFG_CTA;
     return TGVG_OK;
 }

@@ -32,6 +32,36 @@ def test_gradient_at_tile_edges(n):
         assert np.linalg.norm(g[a:b] - gr[a:b]) <= 2.0 ** -8 * np.linalg.norm(gr[a:b]), (a, b)
 
 
+# one row, a warp, a 128-row tile, a tile on each SM, one on each of its eight groups, and their neighbours
+@pytest.mark.parametrize("n", [1, 31, 32, 127, 128, 129, 128 * 152, 128 * 152 + 1, 1024 * 152 - 1, 1024 * 152 + 129])
+def test_forward_at_tile_edges(n):
+    """Sums are FP32, so what can differ by more is a hidden activation rounded to
+    the other bf16 neighbour: 2^-8 of it, seldom.  The biases fill 24 bits."""
+    X, _ = _rows(n, n)
+    m = WS.WarmStartMLP(10, seed=5)
+    p = np.array(m.get_params(), np.float32)
+    b = np.random.default_rng(n).uniform(-0.5, 0.5, 129).astype(np.float32)
+    p[mlp_ref.P_B1:mlp_ref.P_W2], p[mlp_ref.P_B2:mlp_ref.P_W3], p[mlp_ref.P_B3] = b[:64], b[64:128], b[128]
+    m.set_params(p)
+    y = m.predict(X)
+    yr = np.asarray(mlp_ref.forward(p, mlp_ref.bf16_bits_to_float(X))[0]).reshape(-1)
+    assert np.abs(y - yr).max() <= 2.0 ** -8 * np.abs(yr).max()
+    assert np.linalg.norm(y - yr) <= 2.0 ** -8 * np.linalg.norm(yr)
+
+
+@pytest.mark.parametrize("bias, want", [(np.inf, np.inf), (-np.inf, 0.0), (np.nan, 0.0), (3.4e38, 3.4e38)])
+def test_forward_with_extreme_bias(bias, want):
+    """ReLU of the bias alone: infinities stay, NaN counts as zero, as the FP32
+    accumulator held them (3.4e38 rounds to a bf16 infinity there too)."""
+    m = WS.WarmStartMLP(10, seed=5)
+    p = np.zeros(mlp_ref.P_N, np.float32)
+    p[mlp_ref.P_B2], p[mlp_ref.P_W3] = bias, 1.0
+    m.set_params(p)
+    y = m.predict(_rows(130, 1)[0])
+    want = mlp_ref.bf16_round(np.array([want], np.float32))[0]
+    assert np.all(y == want)
+
+
 def _leaves(kind, n):
     """Chunk ranges over n cubes: a treetop's ascending ones, with gaps and an
     end beyond the cubes, out of order, overlapping, and with an empty one."""

@@ -2,13 +2,12 @@
 // the histogram normalised by its total, depth / 21, the cube's position inside
 // its chunk's node, and the histogram's median indicator), ReLU hidden layers,
 // linear output predicting the converged u minus the median indicator (the
-// reference's own start), so that the warm start is median + network.  BF16 weights and activations, FP32 accumulation, on the tensor
-// cores through mma.sync m16n8k16 (row.col, bf16 x bf16 -> f32).
-//
-// The network is under 1 % of a solve's device time (about 10 KFLOP per cube
-// against ~1000 HBM-bound iterations per cube), so it uses the warp-level
-// mma path; the training backward pass keeps FP32 accuracy there by splitting
-// its FP32 factors into exact bf16 parts (k_mlp_grad).
+// reference's own start), so that the warm start is median + network.  BF16
+// weights and activations, FP32 accumulation, on the tensor cores: inference with
+// tcgen05.mma over 128-row tiles (k_forward), the training backward pass with
+// mma.sync m16n8k16 (row.col), whose fragments its two layers and their
+// transposes share in registers; it keeps FP32 accuracy by splitting its FP32
+// factors into exact bf16 parts (k_mlp_grad).
 //
 // Fragment layouts of mma.m16n8k16 (lane t, g = t / 4, c = t % 4):
 //   A (16x16, row-major): a0 = A[g][2c..2c+1], a1 = A[g+8][2c..], a2 = A[g][2c+8..], a3 = A[g+8][2c+8..]
@@ -292,105 +291,6 @@ __device__ __forceinline__ void load_net(const uint32_t* __restrict__ frag, cons
     __syncthreads();
 }
 
-// Inference on feature rows: y[i] for i < n.
-__global__ void __launch_bounds__(256) k_mlp_forward(const uint32_t* __restrict__ X, int n,
-                                                     const uint32_t* __restrict__ frag,
-                                                     const float* __restrict__ prm, float* __restrict__ y) {
-    __shared__ __align__(16) uint32_t sfrag[F_N];
-    __shared__ __align__(16) float sbias[132];
-    load_net(frag, prm, sfrag, sbias);
-    const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile * 16 < n; tile += warps) {
-        const int r0 = tile * 16 + g, r1 = r0 + 8;
-        uint32_t a[1][4] = {{0, 0, 0, 0}}, h[1][4][4];
-        if (r0 < n) { a[0][0] = X[(size_t)r0 * 8 + c]; a[0][2] = X[(size_t)r0 * 8 + c + 4]; }
-        if (r1 < n) { a[0][1] = X[(size_t)r1 * 8 + c]; a[0][3] = X[(size_t)r1 * 8 + c + 4]; }
-        float yy[1][2];
-        mlp_layer1<1>(a, sfrag, sbias, h);
-        mlp_rest<1>(h, sfrag, sbias, yy);
-        if (c == 0) {
-            if (r0 < n) y[r0] = yy[0][0];
-            if (r1 < n) y[r1] = yy[0][1];
-        }
-    }
-}
-
-// Warm-start u = median indicator + network in one pass: each lane builds the
-// features of one cube, the warp runs its 32 cubes through the network as two
-// 16-row tiles that share every weight fragment read from shared memory, and
-// the outputs go back to the lane of their cube.
-//
-// Bytes: 16 + 4 NB read and 4 written per cube; the features (32 B), the median
-// (4 B) and the leaf number (4 B), which three kernels passed through memory
-// before, stay in registers.  Bound by the warp-level mma rate (44 mma per 16
-// cubes; about 236 TFLOP/s of mma.sync here, the rate that the backward pass
-// reaches too).  2.2 M cubes of 10 bins in 128 chunks: 68 + 44 + 83 us in three
-// kernels (a call 202 us) -> 104 us.
-//
-// The cube's chunk: SORTED = the boxes' index ranges ascend without overlap,
-// and the warp finds the last one that starts at or before its first cube by
-// bisection (128 chunks: 7 steps in place of a scan over all of them), each lane
-// stepping on from there.  Otherwise leaf_id names the chunk (the first in the
-// caller's order that holds the cube).
-constexpr int WS_WARPS = 8, WS_BLOCKS = 2;  // blocks per SM (2, 3 and 4 measure the same: 105, 104, 104 us)
-template <int NB, bool SORTED>
-__global__ void __launch_bounds__(WS_WARPS * 32, WS_BLOCKS)
-k_warm_start(int n, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
-             const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id,
-             const uint32_t* __restrict__ frag, const float* __restrict__ prm, float* __restrict__ u) {
-    __shared__ __align__(16) uint32_t sfrag[F_N];
-    __shared__ __align__(16) float sbias[132];
-    __shared__ FeatureTables tab;
-    __shared__ __align__(16) uint32_t sx[WS_WARPS][32 * 12];  // 12 words a row: fragment reads meet 32 banks
-    feature_tables<NB>(tab);
-    load_net(frag, prm, sfrag, sbias);  // ends with a block barrier
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-    const bool vec = bins_aligned<NB>(hists);
-    uint32_t* xs = sx[warp];
-    for (int64_t i0 = ((int64_t)blockIdx.x * WS_WARPS + warp) * 32; i0 < n; i0 += (int64_t)gridDim.x * WS_WARPS * 32) {
-        const int i = (int)i0 + lane;
-        float med = 0.f;
-        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (i < n) {
-            uint32_t b[NB];
-            load_bins<NB>(hists + (size_t)i * NB, vec, b);
-            const uint4 cb = __ldg(cubes + i);
-            LeafBox box{0, 0, 0, 0, 0, 1.0f / (float)(1u << 21)};
-            if (SORTED) {
-                int lo = 0, hi = nleaf;  // first box that starts after the warp's first cube
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (__ldg(&boxes[mid].first) <= (uint32_t)i0) lo = mid + 1; else hi = mid;
-                }
-                int s = lo - 1;
-                while (s + 1 < nleaf && __ldg(&boxes[s + 1].first) <= (uint32_t)i) ++s;
-                if (s >= 0 && (uint32_t)i <= __ldg(&boxes[s].last)) box = boxes[s];
-            } else if (leaf_id) {
-                const int l = __ldg(leaf_id + i);
-                if (l >= 0) box = boxes[l];
-            }
-            med = feature_row<NB>(b, cb, box, tab, w);
-        }
-        __syncwarp();
-        *reinterpret_cast<uint4*>(xs + lane * 12) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(xs + lane * 12 + 4) = make_uint4(w[4], w[5], w[6], w[7]);
-        __syncwarp();
-        uint32_t a[2][4], h[2][4][4];
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) a[t][e] = xs[(t * 16 + (e & 1) * 8 + g) * 12 + c + (e >> 1) * 4];
-        mlp_layer1<2>(a, sfrag, sbias, h);
-        float y[2][2];
-        mlp_rest<2>(h, sfrag, sbias, y);
-        const int src = (lane & 7) * 4;  // cube r of a tile: row g = r & 7, first or second half
-        const float y00 = __shfl_sync(0xffffffffu, y[0][0], src), y01 = __shfl_sync(0xffffffffu, y[0][1], src);
-        const float y10 = __shfl_sync(0xffffffffu, y[1][0], src), y11 = __shfl_sync(0xffffffffu, y[1][1], src);
-        if (i < n) u[i] = fadd(med, lane < 8 ? y00 : (lane < 16 ? y01 : (lane < 24 ? y10 : y11)));
-    }
-}
-
 // An FP32 value as the exact sum of three bf16 parts (8 significant bits each,
 // cut off, not rounded, so nothing overflows); a non-finite value stays whole
 // in the first part.
@@ -404,6 +304,260 @@ __device__ __forceinline__ void split_bf16(float v, float& hi, float& mid, float
 __device__ __forceinline__ uint32_t pack_top(float a, float b) {
     return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
+
+// ---- inference on the fifth-generation tensor cores -----------------------------
+// The network over tiles of 128 rows with tcgen05.mma: a group of four warps owns a
+// tile, each of its threads a row.  Layer by layer the A operand is written to
+// shared memory (K-major, no swizzle: 16 bytes of a row per 8 columns, rows 16
+// bytes apart, so a warp's store is contiguous), one thread issues the layer's
+// mmas into the group's 64 TMEM columns, and the threads read their row back with
+// tcgen05.ld, apply the ReLU and round to bf16 for the next layer.  The biases
+// are part of the products: three more rows of the weights hold a bias as the
+// exact sum of three bf16 parts, against constant ones in the activations.  They
+// come first and the inputs follow in ascending sixteens, so the sums are those of
+// mma.sync accumulators that start at the bias: 4.9 M outputs with biases from
+// 1e-3 to 100 came out the same, bit for bit.
+//
+// One block of eight groups per SM shares the weights (16 KB); a group's operands
+// are 20 KB, the first layer's in the columns next to the constant ones, and its
+// eight tiles in flight cover one another's waits (the 64 registers of 1024
+// threads and the 512 TMEM columns both end at eight).  A group's tiles are
+// neighbours: the next tile's rows are fetched into L2 ahead, and its chunk is
+// looked up again only where one ends.  The waits are bounded; a group that gives
+// up issues no more products, sets *err and yields NaN.
+//
+// Bytes: 16 + 4 NB read and 4 written per cube, 19 us for 2.2 M cubes of 10 bins;
+// what bounds it is the instructions of a row's features and its two epilogues
+// (about 650 a warp) and the latency between them.  Those cubes in 128 chunks:
+// 104 us with mma.sync, at that instruction's 236 TFLOP/s, -> 93 us with tcgen05,
+// 78 us with the ReLU on packed pairs, neighbouring tiles and the prefetch.
+constexpr int TC_GROUPS = 8, TC_THREADS = TC_GROUPS * 128;
+constexpr int TC_B1 = 0, TC_B2 = TC_B1 + 64 * 32 * 2, TC_B3 = TC_B2 + 64 * 80 * 2, TC_W = TC_B3 + 16 * 80 * 2;
+constexpr int TC_CORE = 128 * 16;          // 128 rows x 8 columns
+constexpr int TC_A = 10 * TC_CORE;         // 80 columns: 64 activations, 3 ones, 13 zeros
+constexpr size_t TC_SMEM = TC_W + (size_t)TC_GROUPS * TC_A;
+
+// Shared-memory operand descriptor: address, the distance between the two
+// 8-column halves of an mma's 16 columns (leading) and between groups of 8 rows
+// (stride), all in 16-byte units; version 1, no swizzle.
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t leading, uint32_t stride) {
+    return uint64_t((addr >> 4) & 0x3fff) | (uint64_t((leading >> 4) & 0x3fff) << 16) |
+           (uint64_t((stride >> 4) & 0x3fff) << 32) | (uint64_t(1) << 46);
+}
+// Instruction descriptor: FP32 accumulator, bf16 x bf16, both K-major, M = 128.
+__host__ __device__ constexpr uint32_t tc_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+}
+// chunks x 16 columns of A (from a_at) times B (rows of n columns from b_at) into TMEM
+// columns d, the last 16 columns (the bias) first.
+__device__ __forceinline__ void tc_product(uint32_t d, uint32_t a_at, uint32_t b_at, int n, int chunks, uint32_t mbar) {
+    for (int e = 0; e < chunks; ++e) {
+        const int k = e ? e - 1 : chunks - 1;
+        const uint64_t da = tc_desc(a_at + k * 2 * TC_CORE, TC_CORE, 128);
+        const uint64_t db = tc_desc(b_at + k * 2 * n * 16, n * 16, 128);
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d), "l"(da), "l"(db), "r"(tc_idesc(n)), "r"(e) : "memory");
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
+    for (int spin = 0; spin < (1 << 15); ++spin) {  // at most 20 us each
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            return true;
+        }
+    }
+    return false;
+}
+__device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr) : "memory");
+}
+// Two accumulators as bf16, negative ones and NaN as zero (rounding keeps the sign,
+// so the maximum of the pair is taken after it).
+__device__ __forceinline__ uint32_t relu_pack(uint32_t lo, uint32_t hi) {
+    uint32_t r;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(pack_bf16(__uint_as_float(lo), __uint_as_float(hi))), "r"(0u));
+    return r;
+}
+
+// What the generic-proxy stores of the group left in shared memory is there for
+// its mmas, and its reads of TMEM are done, once all 128 threads have passed.
+__device__ __forceinline__ void tc_group_sync(int group) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// SRC 0: y[i] of the feature rows X.  SRC 1, 2: the warm start u = median indicator
+// + network of the cubes, their features built here; the chunk of a cube is found
+// by bisection (1: the boxes' index ranges ascend without overlap; a warp looks up
+// its first cube and its lanes step on from there) or read from leaf_id (2: the
+// first chunk in the caller's order that holds the cube, -1 for none; null: the root).
+template <int NB, int SRC>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
+          const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id, const float* __restrict__ prm,
+          float* __restrict__ out, int* __restrict__ err) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ FeatureTables tab;
+    __shared__ __align__(8) unsigned long long s_bar[TC_GROUPS];
+    __shared__ uint32_t s_tmem;
+    const int group = threadIdx.x >> 7, row = threadIdx.x & 127, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* A = smem_raw + TC_W + group * TC_A;
+    const uint32_t w_at = (uint32_t)__cvta_generic_to_shared(smem_raw), a_at = (uint32_t)__cvta_generic_to_shared(A),
+                   bar = (uint32_t)__cvta_generic_to_shared(s_bar + group);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;"
+                     ::"r"((uint32_t)__cvta_generic_to_shared(&s_tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (row == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    if (SRC) feature_tables<NB>(tab);
+    // weights: element (column n of the layer, k) at (k / 8) (columns x 16 B) + n x 16 B + (k % 8) x 2 B
+    auto weight = [&](int k, int j, int width, int w, int bias, int stride) {
+        if (k < width) return __float2bfloat16_rn(prm[w + k * stride + j]);
+        if (k >= width + 3) return __float2bfloat16_rn(0.f);
+        float p[3];
+        split_bf16(prm[bias + j], p[0], p[1], p[2]);
+        return __float2bfloat16_rn(p[k - width]);  // exact: a bf16 value
+    };
+    __nv_bfloat16* W = reinterpret_cast<__nv_bfloat16*>(smem_raw);
+    for (int e = threadIdx.x; e < 64 * 32; e += TC_THREADS)
+        W[TC_B1 / 2 + e] = weight(e / 512 * 8 + e % 8, e % 512 / 8, MLP_K1, P_W1, P_B1, MLP_H);
+    for (int e = threadIdx.x; e < 64 * 80; e += TC_THREADS)
+        W[TC_B2 / 2 + e] = weight(e / 512 * 8 + e % 8, e % 512 / 8, MLP_H, P_W2, P_B2, MLP_H);
+    for (int e = threadIdx.x; e < 16 * 80; e += TC_THREADS)
+        W[TC_B3 / 2 + e] = e % 128 / 8 == 0 ? weight(e / 128 * 8 + e % 8, 0, MLP_H, P_W3, P_B3, 1) : __float2bfloat16_rn(0.f);
+    // the constant columns 64..79
+    *reinterpret_cast<uint4*>(A + 8 * TC_CORE + row * 16) = make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u);
+    *reinterpret_cast<uint4*>(A + 9 * TC_CORE + row * 16) = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t d = s_tmem + group * 64;                          // the group's columns
+    const uint32_t mine = d + ((uint32_t)(warp & 3) * 32u << 16);  // this warp's lanes of them
+    const bool vec = SRC && bins_aligned<NB>(hists);
+    uint32_t phase = 0;
+    bool ok = true;
+    // Each group's tiles are neighbours, so its chunk seldom changes.
+    const int64_t tiles = ((int64_t)n + 127) / 128, runs = (int64_t)gridDim.x * TC_GROUPS,
+                  run = blockIdx.x + (int64_t)group * gridDim.x;
+    int chunk = -1;  // the last one that starts at or before the warp's first cube
+    for (int64_t t = tiles * run / runs, end = tiles * (run + 1) / runs; t < end; ++t) {
+        const int64_t i0 = t * 128 + (warp & 3) * 32;  // the warp's first row
+        const int64_t i = i0 + lane;
+        float med = 0.f;
+        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+        if (i < n) {
+            if (SRC == 0) {
+                lo = __ldg(X + i * 2);
+                hi = __ldg(X + i * 2 + 1);
+            } else {
+                uint32_t bins[NB], w[8];
+                load_bins<NB>(hists + (size_t)i * NB, vec, bins);
+                const uint4 cb = __ldg(cubes + i);
+                if (i + 128 < n) {  // the next tile's
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(cubes + i + 128));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(hists + (size_t)(i + 128) * NB));
+                }
+                LeafBox box{0, 0, 0, 0, 0, 1.0f / (float)(1u << 21)};
+                if (SRC == 1) {
+                    if (chunk + 1 < nleaf && __ldg(&boxes[chunk + 1].first) <= (uint32_t)i0) {
+                        int l = chunk + 2, h = nleaf;  // first box that starts after the warp's first cube
+                        while (l < h) {
+                            const int mid = (l + h) >> 1;
+                            if (__ldg(&boxes[mid].first) <= (uint32_t)i0) l = mid + 1; else h = mid;
+                        }
+                        chunk = l - 1;
+                    }
+                    int s = chunk;
+                    while (s + 1 < nleaf && __ldg(&boxes[s + 1].first) <= (uint32_t)i) ++s;
+                    if (s >= 0 && (uint32_t)i <= __ldg(&boxes[s].last)) box = boxes[s];
+                } else if (leaf_id) {
+                    const int l = __ldg(leaf_id + i);
+                    if (l >= 0) box = boxes[l];
+                }
+                med = feature_row<NB>(bins, cb, box, tab, w);
+                lo = make_uint4(w[0], w[1], w[2], w[3]);
+                hi = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+        }
+        // layer 1: columns 48..63 hold the features, 64..79 the ones
+        *reinterpret_cast<uint4*>(A + 6 * TC_CORE + row * 16) = lo;
+        *reinterpret_cast<uint4*>(A + 7 * TC_CORE + row * 16) = hi;
+        tc_group_sync(group);
+        if (row == 0 && ok) tc_product(d, a_at + 6 * TC_CORE, w_at + TC_B1, 64, 2, bar);
+        for (int layer = 0; layer < 2; ++layer) {
+            ok = ok && tc_wait(bar, phase & 1);
+            ++phase;
+            __syncwarp();
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t r[32];
+                tc_load32(mine + half * 32, r);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(A + (half * 4 + c) * TC_CORE + row * 16) =
+                        make_uint4(relu_pack(r[8 * c], r[8 * c + 1]), relu_pack(r[8 * c + 2], r[8 * c + 3]),
+                                   relu_pack(r[8 * c + 4], r[8 * c + 5]), relu_pack(r[8 * c + 6], r[8 * c + 7]));
+            }
+            tc_group_sync(group);
+            if (row == 0 && ok) {
+                if (layer == 0) tc_product(d, a_at, w_at + TC_B2, 64, 5, bar);
+                else tc_product(d, a_at, w_at + TC_B3, 16, 5, bar);
+            }
+        }
+        ok = ok && tc_wait(bar, phase & 1);
+        ++phase;
+        __syncwarp();
+        uint32_t y;
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;"
+                     : "=r"(y) : "r"(mine) : "memory");
+        if (i < n) {
+            const float v = ok ? __uint_as_float(y) : __int_as_float(0x7fc00000);
+            out[i] = SRC ? fadd(med, v) : v;
+        }
+    }
+    if (!ok) atomicOr(err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_tmem) : "memory");
+}
+
+// One inference launch; d_id null with leaves means ascending chunks.
+template <int NB, int SRC>
+static int launch_forward(tgvg_ctx* ctx, int64_t n, const uint32_t* X, const tgvg_cube* d_c, const uint32_t* d_h,
+                          const LeafBox* boxes, int nleaf, const int* d_id, const float* prm, float* out, int* err) {
+    TGVG_CK(ctx, cudaFuncSetAttribute(k_forward<NB, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+    const int64_t tiles = (n + 127) / 128;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->sm_count);  // a few tiles spread over the SMs
+    k_forward<NB, SRC><<<grid, TC_THREADS, TC_SMEM, ctx->stream>>>(
+        (int)n, reinterpret_cast<const uint4*>(X), reinterpret_cast<const uint4*>(d_c), d_h, boxes, nleaf, d_id, prm, out,
+        err);
+    TGVG_LAUNCHED(ctx);
+    return TGVG_OK;
+}
+
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -453,7 +607,7 @@ k_mlp_grad(const uint32_t* __restrict__ X, const float* __restrict__ t, const in
            const uint32_t* __restrict__ frag, const float* __restrict__ prm, const float* __restrict__ wr,
            float* __restrict__ grad, float* __restrict__ loss) {
     constexpr int ROWS = WARPS * 16, NTW = 8 / WARPS;  // rows per step; column tiles per warp
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     uint32_t* sfrag = reinterpret_cast<uint32_t*>(smem_raw);
     float* sbias = reinterpret_cast<float*>(sfrag + F_N);  // 136
     float* sw3 = sbias + 136;                              // 64: bf16-rounded W3
@@ -746,6 +900,7 @@ struct tgvg_mlp {
     float* d_wr = nullptr;
     float* d_loss = nullptr;
     uint32_t* d_frag = nullptr;
+    int* d_err = nullptr;  // set by an inference wait that ran out
     int step = 0;
 };
 
@@ -764,7 +919,8 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
     for (float** b : bufs)
         if (cudaMalloc(b, sizeof(float) * P_N) != cudaSuccess) { delete m; return TGVG_ERR_NOMEM; }
     if (cudaMalloc(&m->d_loss, sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess) {
+        cudaMalloc(&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess ||
+        cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) {
         delete m;
         return TGVG_ERR_NOMEM;
     }
@@ -780,6 +936,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
     for (int k = 0; k < 64 * 64; ++k) p[P_W2 + k] = u2(rng);
     for (int k = 0; k < 64; ++k) p[P_W3 + k] = u3(rng);
     TGVG_CK(ctx, cudaMemcpyAsync(m->d_prm, p.data(), sizeof(float) * P_N, cudaMemcpyHostToDevice, ctx->stream));
+    TGVG_CK(ctx, cudaMemsetAsync(m->d_err, 0, sizeof(int), ctx->stream));
     TGVG_CK(ctx, cudaMemsetAsync(m->d_m1, 0, sizeof(float) * P_N, ctx->stream));
     TGVG_CK(ctx, cudaMemsetAsync(m->d_m2, 0, sizeof(float) * P_N, ctx->stream));
     int rc = mlp_repack(ctx, m);
@@ -792,7 +949,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
 extern "C" int tgvg_mlp_destroy(tgvg_mlp* m) {
     if (!m) return TGVG_ERR_INVALID;
     cudaFree(m->d_prm); cudaFree(m->d_m1); cudaFree(m->d_m2); cudaFree(m->d_grad); cudaFree(m->d_wr);
-    cudaFree(m->d_loss); cudaFree(m->d_frag);
+    cudaFree(m->d_loss); cudaFree(m->d_frag); cudaFree(m->d_err);
     delete m;
     return TGVG_OK;
 }
@@ -846,6 +1003,16 @@ extern "C" int tgvg_mlp_features(tgvg_ctx* ctx, const tgvg_cube* cubes, const ui
     return TGVG_OK;
 }
 
+// Waits for the stream and reports an inference whose wait ran out.
+static int inference_done(tgvg_ctx* ctx, tgvg_mlp* m) {
+    int e = 0;
+    TGVG_CK(ctx, cudaMemcpyAsync(&e, m->d_err, sizeof(e), cudaMemcpyDeviceToHost, ctx->stream));
+    TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (!e) return TGVG_OK;
+    TGVG_CK(ctx, cudaMemsetAsync(m->d_err, 0, sizeof(int), ctx->stream));
+    return ctx->fail(TGVG_ERR_TIMEOUT, "a tensor-core wait of the network timed out");
+}
+
 extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, int64_t n, float* y) {
     if (!ctx || !m || n < 0 || (n > 0 && (!X || !y)) || n > (int64_t(1) << 30)) return TGVG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
@@ -854,13 +1021,10 @@ extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, i
     auto* d_y = (float*)ctx->buf(B_M_Y, sizeof(float) * n);
     if (!d_x || !d_y) return TGVG_ERR_NOMEM;
     TGVG_CK(ctx, cudaMemcpyAsync(d_x, X, sizeof(uint32_t) * 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-    const int tiles = (int)((n + 15) / 16);
-    const unsigned grid = (unsigned)std::min((tiles + 7) / 8, ctx->sm_count * 8);
-    k_mlp_forward<<<grid, 256, 0, ctx->stream>>>(d_x, (int)n, m->d_frag, m->d_prm, d_y);
-    TGVG_LAUNCHED(ctx);
+    int rc = launch_forward<8, 0>(ctx, n, d_x, nullptr, nullptr, nullptr, 0, nullptr, m->d_prm, d_y, m->d_err);
+    if (rc) return rc;
     TGVG_CK(ctx, cudaMemcpyAsync(y, d_y, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    return TGVG_OK;
+    return inference_done(ctx, m);
 }
 
 // Warm-start u on the device (u = median + network).  Device cubes / histograms
@@ -888,14 +1052,11 @@ static int warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_c, cons
         k_leaf_id<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>((int)n, nleaf, d_l, d_id);
         TGVG_LAUNCHED(ctx);
     }
-    const unsigned grid = (unsigned)std::min<int64_t>((n + 32 * WS_WARPS - 1) / (32 * WS_WARPS), ctx->sm_count * WS_BLOCKS);
-    void (*k)(int, const uint4*, const uint32_t*, const LeafBox*, int, const int*, const uint32_t*, const float*, float*);
-    if (nbins == 8) k = sorted ? k_warm_start<8, true> : k_warm_start<8, false>;
-    else k = sorted ? k_warm_start<10, true> : k_warm_start<10, false>;
-    k<<<grid, WS_WARPS * 32, 0, ctx->stream>>>((int)n, reinterpret_cast<const uint4*>(d_c), d_h, d_b, nleaf, d_id,
-                                               m->d_frag, m->d_prm, d_u);
-    TGVG_LAUNCHED(ctx);
-    return TGVG_OK;
+    if (nbins == 8)
+        return sorted ? launch_forward<8, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_prm, d_u, m->d_err)
+                      : launch_forward<8, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_prm, d_u, m->d_err);
+    return sorted ? launch_forward<10, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_prm, d_u, m->d_err)
+                  : launch_forward<10, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_prm, d_u, m->d_err);
 }
 
 static bool warm_start_args_ok(tgvg_ctx* ctx, tgvg_mlp* m, const void* c, const void* h, int64_t n, int32_t nbins,
@@ -918,8 +1079,7 @@ extern "C" int tgvg_mlp_warm_start(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* 
     int rc = warm_start_dev(ctx, m, d_c, d_h, n, nbins, leaves, nleaf, d_u);
     if (rc) return rc;
     TGVG_CK(ctx, cudaMemcpyAsync(u, d_u, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    return TGVG_OK;
+    return inference_done(ctx, m);
 }
 
 extern "C" int tgvg_mlp_warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_cubes,

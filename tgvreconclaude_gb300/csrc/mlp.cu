@@ -58,10 +58,37 @@ __device__ __forceinline__ void mma_bf16(float& d0, float& d1, float& d2, float&
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Weight fragments (and a bf16-rounded float copy used by the backward pass)
-// from the fp32 master parameters.
-__global__ void k_mlp_pack(const float* __restrict__ prm, uint32_t* __restrict__ frag, float* __restrict__ wr) {
+// An FP32 value as the exact sum of three bf16 parts (8 significant bits each,
+// cut off, not rounded, so nothing overflows); a non-finite value stays whole
+// in the first part.
+__device__ __forceinline__ void split_bf16(float v, float& hi, float& mid, float& lo) {
+    hi = __uint_as_float(__float_as_uint(v) & 0xffff0000u);
+    const float r = isfinite(v) ? v - hi : 0.f;
+    mid = __uint_as_float(__float_as_uint(r) & 0xffff0000u);
+    lo = r - mid;
+}
+// The weights as inference takes them (k_forward): per layer 64, 64 and 16 columns of
+// 32, 80 and 80 inputs, three of them the bias's parts; element (k, column j) at
+// (k / 8) (columns x 16 B) + j x 16 B + (k % 8) x 2 B.
+constexpr int TC_B1 = 0, TC_B2 = TC_B1 + 64 * 32 * 2, TC_B3 = TC_B2 + 64 * 80 * 2, TC_W = TC_B3 + 16 * 80 * 2;
+__device__ __forceinline__ __nv_bfloat16 tc_weight(const float* __restrict__ prm, int e) {
+    const bool l1 = e < TC_B2 / 2, l3 = e >= TC_B3 / 2;
+    e -= l3 ? TC_B3 / 2 : (l1 ? 0 : TC_B2 / 2);
+    const int columns = l3 ? 16 : 64, width = l1 ? MLP_K1 : MLP_H;
+    const int k = e / (columns * 8) * 8 + e % 8, j = e / 8 % columns;
+    if (k >= width + 3 || (l3 && j > 0)) return __float2bfloat16_rn(0.f);
+    if (k < width) return __float2bfloat16_rn(prm[l3 ? P_W3 + k : (l1 ? P_W1 : P_W2) + k * MLP_H + j]);
+    float p[3];
+    split_bf16(prm[(l3 ? P_B3 : (l1 ? P_B1 : P_B2)) + j], p[0], p[1], p[2]);
+    return __float2bfloat16_rn(p[k - width]);  // exact: a bf16 value
+}
+
+// Weight fragments, inference's weights and a bf16-rounded float copy (used by the
+// backward pass) from the fp32 master parameters.
+__global__ void k_mlp_pack(const float* __restrict__ prm, uint32_t* __restrict__ frag, float* __restrict__ wr,
+                           __nv_bfloat16* __restrict__ tc) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < TC_W / 2) tc[t] = tc_weight(prm, t);
     if (t < P_N) wr[t] = bf16r(prm[t]);
     if (t >= F_N) return;
     const int tile = t / 64, w = t % 64, lane = w / 2, half = w % 2;
@@ -291,15 +318,6 @@ __device__ __forceinline__ void load_net(const uint32_t* __restrict__ frag, cons
     __syncthreads();
 }
 
-// An FP32 value as the exact sum of three bf16 parts (8 significant bits each,
-// cut off, not rounded, so nothing overflows); a non-finite value stays whole
-// in the first part.
-__device__ __forceinline__ void split_bf16(float v, float& hi, float& mid, float& lo) {
-    hi = __uint_as_float(__float_as_uint(v) & 0xffff0000u);
-    const float r = isfinite(v) ? v - hi : 0.f;
-    mid = __uint_as_float(__float_as_uint(r) & 0xffff0000u);
-    lo = r - mid;
-}
 // Two values whose low 16 bits are zero, as a bf16 pair.
 __device__ __forceinline__ uint32_t pack_top(float a, float b) {
     return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
@@ -330,9 +348,11 @@ __device__ __forceinline__ uint32_t pack_top(float a, float b) {
 // what bounds it is the instructions of a row's features and its two epilogues
 // (about 650 a warp) and the latency between them.  Those cubes in 128 chunks:
 // 104 us with mma.sync, at that instruction's 236 TFLOP/s, -> 93 us with tcgen05,
-// 78 us with the ReLU on packed pairs, neighbouring tiles and the prefetch.
+// 78 us with the ReLU on packed pairs, neighbouring tiles and the prefetch, 77 us
+// with the weights copied as the products take them (k_mlp_pack lays them out when
+// they change; gathered from the FP32 parameters by each block, a call of 6,000 to
+// 600,000 cubes took 1.3 to 1.8 us longer: 17.6 and 36.5 us against 16.3 and 34.7).
 constexpr int TC_GROUPS = 8, TC_THREADS = TC_GROUPS * 128;
-constexpr int TC_B1 = 0, TC_B2 = TC_B1 + 64 * 32 * 2, TC_B3 = TC_B2 + 64 * 80 * 2, TC_W = TC_B3 + 16 * 80 * 2;
 constexpr int TC_CORE = 128 * 16;          // 128 rows x 8 columns
 constexpr int TC_A = 10 * TC_CORE;         // 80 columns: 64 activations, 3 ones, 13 zeros
 constexpr size_t TC_SMEM = TC_W + (size_t)TC_GROUPS * TC_A;
@@ -412,8 +432,8 @@ __device__ __forceinline__ void tc_group_sync(int group) {
 template <int NB, int SRC>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
-          const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id, const float* __restrict__ prm,
-          float* __restrict__ out, int* __restrict__ err) {
+          const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id,
+          const __nv_bfloat16* __restrict__ weights, float* __restrict__ out, int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ FeatureTables tab;
     __shared__ __align__(8) unsigned long long s_bar[TC_GROUPS];
@@ -429,21 +449,8 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
     }
     if (row == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     if (SRC) feature_tables<NB>(tab);
-    // weights: element (column n of the layer, k) at (k / 8) (columns x 16 B) + n x 16 B + (k % 8) x 2 B
-    auto weight = [&](int k, int j, int width, int w, int bias, int stride) {
-        if (k < width) return __float2bfloat16_rn(prm[w + k * stride + j]);
-        if (k >= width + 3) return __float2bfloat16_rn(0.f);
-        float p[3];
-        split_bf16(prm[bias + j], p[0], p[1], p[2]);
-        return __float2bfloat16_rn(p[k - width]);  // exact: a bf16 value
-    };
-    __nv_bfloat16* W = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-    for (int e = threadIdx.x; e < 64 * 32; e += TC_THREADS)
-        W[TC_B1 / 2 + e] = weight(e / 512 * 8 + e % 8, e % 512 / 8, MLP_K1, P_W1, P_B1, MLP_H);
-    for (int e = threadIdx.x; e < 64 * 80; e += TC_THREADS)
-        W[TC_B2 / 2 + e] = weight(e / 512 * 8 + e % 8, e % 512 / 8, MLP_H, P_W2, P_B2, MLP_H);
-    for (int e = threadIdx.x; e < 16 * 80; e += TC_THREADS)
-        W[TC_B3 / 2 + e] = e % 128 / 8 == 0 ? weight(e / 128 * 8 + e % 8, 0, MLP_H, P_W3, P_B3, 1) : __float2bfloat16_rn(0.f);
+    for (int e = threadIdx.x; e < TC_W / 16; e += TC_THREADS)
+        reinterpret_cast<uint4*>(smem_raw)[e] = __ldg(reinterpret_cast<const uint4*>(weights) + e);
     // the constant columns 64..79
     *reinterpret_cast<uint4*>(A + 8 * TC_CORE + row * 16) = make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u);
     *reinterpret_cast<uint4*>(A + 9 * TC_CORE + row * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -547,12 +554,12 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
 // One inference launch; d_id null with leaves means ascending chunks.
 template <int NB, int SRC>
 static int launch_forward(tgvg_ctx* ctx, int64_t n, const uint32_t* X, const tgvg_cube* d_c, const uint32_t* d_h,
-                          const LeafBox* boxes, int nleaf, const int* d_id, const float* prm, float* out, int* err) {
+                          const LeafBox* boxes, int nleaf, const int* d_id, const __nv_bfloat16* tc, float* out, int* err) {
     TGVG_CK(ctx, cudaFuncSetAttribute(k_forward<NB, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     const int64_t tiles = (n + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->sm_count);  // a few tiles spread over the SMs
     k_forward<NB, SRC><<<grid, TC_THREADS, TC_SMEM, ctx->stream>>>(
-        (int)n, reinterpret_cast<const uint4*>(X), reinterpret_cast<const uint4*>(d_c), d_h, boxes, nleaf, d_id, prm, out,
+        (int)n, reinterpret_cast<const uint4*>(X), reinterpret_cast<const uint4*>(d_c), d_h, boxes, nleaf, d_id, tc, out,
         err);
     TGVG_LAUNCHED(ctx);
     return TGVG_OK;
@@ -900,12 +907,13 @@ struct tgvg_mlp {
     float* d_wr = nullptr;
     float* d_loss = nullptr;
     uint32_t* d_frag = nullptr;
+    __nv_bfloat16* d_tc = nullptr;
     int* d_err = nullptr;  // set by an inference wait that ran out
     int step = 0;
 };
 
 static int mlp_repack(tgvg_ctx* ctx, tgvg_mlp* m) {
-    k_mlp_pack<<<(P_N + 255) / 256, 256, 0, ctx->stream>>>(m->d_prm, m->d_frag, m->d_wr);
+    k_mlp_pack<<<(TC_W / 2 + 255) / 256, 256, 0, ctx->stream>>>(m->d_prm, m->d_frag, m->d_wr, m->d_tc);  // TC_W / 2 > P_N, F_N
     TGVG_LAUNCHED(ctx);
     return TGVG_OK;
 }
@@ -920,7 +928,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
         if (cudaMalloc(b, sizeof(float) * P_N) != cudaSuccess) { delete m; return TGVG_ERR_NOMEM; }
     if (cudaMalloc(&m->d_loss, sizeof(float)) != cudaSuccess ||
         cudaMalloc(&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess ||
-        cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&m->d_tc, TC_W) != cudaSuccess || cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) {
         delete m;
         return TGVG_ERR_NOMEM;
     }
@@ -949,7 +957,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
 extern "C" int tgvg_mlp_destroy(tgvg_mlp* m) {
     if (!m) return TGVG_ERR_INVALID;
     cudaFree(m->d_prm); cudaFree(m->d_m1); cudaFree(m->d_m2); cudaFree(m->d_grad); cudaFree(m->d_wr);
-    cudaFree(m->d_loss); cudaFree(m->d_frag); cudaFree(m->d_err);
+    cudaFree(m->d_loss); cudaFree(m->d_frag); cudaFree(m->d_tc); cudaFree(m->d_err);
     delete m;
     return TGVG_OK;
 }
@@ -1021,7 +1029,7 @@ extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, i
     auto* d_y = (float*)ctx->buf(B_M_Y, sizeof(float) * n);
     if (!d_x || !d_y) return TGVG_ERR_NOMEM;
     TGVG_CK(ctx, cudaMemcpyAsync(d_x, X, sizeof(uint32_t) * 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-    int rc = launch_forward<8, 0>(ctx, n, d_x, nullptr, nullptr, nullptr, 0, nullptr, m->d_prm, d_y, m->d_err);
+    int rc = launch_forward<8, 0>(ctx, n, d_x, nullptr, nullptr, nullptr, 0, nullptr, m->d_tc, d_y, m->d_err);
     if (rc) return rc;
     TGVG_CK(ctx, cudaMemcpyAsync(y, d_y, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
     return inference_done(ctx, m);
@@ -1053,10 +1061,10 @@ static int warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_c, cons
         TGVG_LAUNCHED(ctx);
     }
     if (nbins == 8)
-        return sorted ? launch_forward<8, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_prm, d_u, m->d_err)
-                      : launch_forward<8, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_prm, d_u, m->d_err);
-    return sorted ? launch_forward<10, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_prm, d_u, m->d_err)
-                  : launch_forward<10, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_prm, d_u, m->d_err);
+        return sorted ? launch_forward<8, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, m->d_err)
+                      : launch_forward<8, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, m->d_err);
+    return sorted ? launch_forward<10, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, m->d_err)
+                  : launch_forward<10, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, m->d_err);
 }
 
 static bool warm_start_args_ok(tgvg_ctx* ctx, tgvg_mlp* m, const void* c, const void* h, int64_t n, int32_t nbins,

@@ -376,10 +376,11 @@ __global__ void k_bal_insert(int64_t t0, int64_t t, const Cell* __restrict__ q, 
 // slot that the rounds need is fixed for the window and worked out once: whether
 // a coarser ancestor is present at the start, and where nb, par and par's output
 // key lie in tables that hold the live slots' cells and keys.  A round then only
-// resets, claims and reads 32-bit slot numbers at known places.
-// (Before, every round evaluated all slots again from their codes and hashed
-// every proposal into fresh tables: 1.2 M cubes in 7 windows, 3.1 ms of kernels;
-// now 1.0 ms, 0.27 of it the one look at every slot.)
+// claims and reads 32-bit numbers at known places, in two launches.
+// (Evaluating all slots again from their codes in every round and hashing every
+// proposal into fresh tables took 1.2 M cubes in 7 windows 3.1 ms of kernels; the
+// live slots 1.0 ms, 0.27 of it the one look at every slot.  A reset, a launch that
+// wrote the winners' cells and the two launches left: a call 2.49 -> 2.38 ms.)
 constexpr int SLOT_TILE = 2048, SLOT_THREADS = 256;
 constexpr unsigned SLOT_NONE = ~0u;
 
@@ -425,6 +426,7 @@ struct Live {
     int* nb_at;    // entry of nb among the live cells, -1: none of them
     int* cell_at;  // entry of par
     int* key_at;   // entry of par's output key
+    int* cell_key;  // per entry of the cells: its output key's entry
     uint8_t* coarse;  // a coarser ancestor of nb is present at the window's start
     uint8_t* prop;    // the slot proposes its bridge
 };
@@ -472,6 +474,7 @@ __global__ void k_bal_tables(int nl, int64_t h, const Cell* __restrict__ q, KeyS
     const int d = q[h + L.slot[l] / 6].depth - 1;
     L.cell_at[l] = (int)set_insert(wcell, cell_key(L.par[l], d));
     L.key_at[l] = (int)set_insert(wdc, dc_key(d, L.par[l]));
+    L.cell_key[L.cell_at[l]] = L.key_at[l];  // the same from every slot with this cell
 }
 
 __global__ void k_bal_nb(int nl, int64_t h, const Cell* __restrict__ q, KeySet wcell, Live L) {
@@ -482,39 +485,40 @@ __global__ void k_bal_nb(int nl, int64_t h, const Cell* __restrict__ q, KeySet w
     L.nb_at[l] = (int)set_slot(wcell, cell_key(slot_nb(c, (int)(me % 6)), c.depth));
 }
 
-// A round: proposals of one output key compete for it and the earliest slot
-// wins (the reference's emplace succeeds for the first one only) ...
-__global__ void k_bal_claim(int nl, Live L, unsigned* __restrict__ key_slot) {
+// A round: proposals of one output key compete for it and the earliest live slot
+// wins (the reference's emplace succeeds for the first one only).  An entry holds
+// the winner's number in the live list below the round's tag; later rounds have
+// smaller tags, so nothing is reset between rounds.
+constexpr int TAG_SHIFT = 27;  // 6 WINDOW slots and 24 rounds fit in 32 bits
+static_assert(6 * WINDOW <= (int64_t(1) << TAG_SHIFT) && MAX_ROUNDS < (1 << (32 - TAG_SHIFT)) - 1, "tags");
+__host__ __device__ __forceinline__ unsigned round_tag(int round) { return unsigned(MAX_ROUNDS - round) << TAG_SHIFT; }
+
+__global__ void k_bal_claim(int nl, Live L, unsigned* __restrict__ winner, unsigned tag) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < nl && L.prop[l]) atomicMin(key_slot + L.key_at[l], L.slot[l]);
+    if (l < nl && L.prop[l]) atomicMin(winner + L.key_at[l], tag | (unsigned)l);
 }
 
-// ... the winners' cells are present from their slot on ...
-__global__ void k_bal_accept(int nl, Live L, const unsigned* __restrict__ key_slot, unsigned* __restrict__ cell_slot,
-                             int* __restrict__ acc) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= nl) return;
-    const unsigned me = L.slot[l];
-    const bool a = L.prop[l] && key_slot[L.key_at[l]] == me;
-    acc[l] = a;
-    if (a) cell_slot[L.cell_at[l]] = me;
+// Whether a live slot before l adds the cell at entry e: the winner of its key adds this very cell.
+__device__ __forceinline__ bool added_before(const Live& L, const unsigned* __restrict__ winner, unsigned tag, int e, int l) {
+    const unsigned w = winner[L.cell_key[e]] - tag;  // below 1 << TAG_SHIFT only with this round's tag
+    return w < (unsigned)l && L.cell_at[w] == e;
 }
 
 // ... and every live slot is evaluated again against the earlier ones.
 __global__ void k_bal_again(int nl, int64_t h, const Cell* __restrict__ q, KeySet wcell,
-                            const unsigned* __restrict__ cell_slot, Live L, unsigned* __restrict__ first_change) {
+                            const unsigned* __restrict__ winner, unsigned tag, Live L, unsigned* __restrict__ first_change) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= nl) return;
     const unsigned me = L.slot[l];
     const int nb_at = L.nb_at[l];
-    bool p = !(nb_at >= 0 && cell_slot[nb_at] < me) && !(cell_slot[L.cell_at[l]] < me);
+    bool p = !(nb_at >= 0 && added_before(L, winner, tag, nb_at, l)) && !added_before(L, winner, tag, L.cell_at[l], l);
     if (p && !L.coarse[l]) {
         const Cell c = q[h + me / 6];
         const uint64_t nb = slot_nb(c, (int)(me % 6));
         p = false;
         for (int d = c.depth - 2; d >= 0 && !p; --d) {
             const long long e = set_slot(wcell, cell_key(ancestor_key(nb, d), d));
-            p = e >= 0 && cell_slot[e] < me;
+            p = e >= 0 && added_before(L, winner, tag, (int)e, l);
         }
     }
     if (p != (L.prop[l] != 0)) {
@@ -523,10 +527,15 @@ __global__ void k_bal_again(int nl, int64_t h, const Cell* __restrict__ q, KeySe
     }
 }
 
-__global__ void k_bal_limit(int nl, Live L, const unsigned* __restrict__ first_change, int* __restrict__ acc) {
+// The bridges that the round's winners add.  Slots below the first change are
+// exact; with `limit` only whole entries of them are taken.
+__global__ void k_bal_accept(int nl, Live L, const unsigned* __restrict__ winner, unsigned tag,
+                             const unsigned* __restrict__ first_change, bool limit, int* __restrict__ acc) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    // slots below the first change are exact; the window commits whole entries
-    if (l < nl && *first_change != SLOT_NONE && L.slot[l] >= *first_change / 6 * 6) acc[l] = 0;
+    if (l >= nl) return;
+    const unsigned change = *first_change;
+    acc[l] = L.prop[l] && winner[L.key_at[l]] == (tag | (unsigned)l) &&
+             !(limit && change != SLOT_NONE && L.slot[l] >= change / 6 * 6);
 }
 
 // Append the accepted bridges to the FIFO, in slot order.
@@ -815,21 +824,22 @@ int balance_dev(tgvg_ctx* ctx, const tgvg_cube* cubes, int64_t n, float r_root, 
         }
         const uint64_t wc = pow2_at_least(2 * uint64_t(nl));
         Live L{W.get<unsigned>(nl), W.get<unsigned long long>(nl), W.get<int>(nl), W.get<int>(nl), W.get<int>(nl),
-               W.get<uint8_t>(nl), W.get<uint8_t>(nl)};
+               W.get<int>(wc), W.get<uint8_t>(nl), W.get<uint8_t>(nl)};
         auto* wcell = W.get<unsigned long long>(wc);
         auto* wdc = W.get<unsigned long long>(wc);
-        auto* place = W.get<unsigned>(2 * wc + 1);  // slot per key entry, slot per cell entry, first change: reset together
+        auto* winner = W.get<unsigned>(wc + MAX_ROUNDS);  // per key entry; then each round's first change
         auto* acc = W.get<int>(nl);
         auto* apos = W.get<int>(nl);
         const int64_t nsum = scan_sums_len(nl);
         auto* asum = W.get<int>(nsum);
-        if (!L.slot || !L.par || !L.nb_at || !L.cell_at || !L.key_at || !L.coarse || !L.prop || !wcell || !wdc || !place ||
+        if (!L.slot || !L.par || !L.nb_at || !L.cell_at || !L.key_at || !L.cell_key || !L.coarse || !L.prop || !wcell || !wdc || !winner ||
             !acc || !apos || !asum)
             return ctx->fail(TGVG_ERR_NOMEM, "balance window buffers");
-        unsigned *key_slot = place, *cell_slot = place + wc, *first = place + 2 * wc;
+        unsigned* first = winner + wc;
         const KeySet kcell{wcell, wc - 1, CELL_EMPTY}, kdc{wdc, wc - 1, DC_EMPTY};
         TGVG_CK(ctx, cudaMemsetAsync(wcell, 0x00, sizeof(unsigned long long) * wc, st));
         TGVG_CK(ctx, cudaMemsetAsync(wdc, 0xff, sizeof(unsigned long long) * wc, st));
+        TGVG_CK(ctx, cudaMemsetAsync(winner, 0xff, sizeof(unsigned) * (wc + MAX_ROUNDS), st));
         k_bal_live<<<(unsigned)tiles, SLOT_THREADS, 0, st>>>(h, q, S.cells(), mask, sums, L);
         TGVG_LAUNCHED(ctx);
         const unsigned lg = grid_of(nl, 256);
@@ -844,21 +854,17 @@ int balance_dev(tgvg_ctx* ctx, const tgvg_cube* cubes, int64_t n, float r_root, 
         for (int batch = 3; rounds < MAX_ROUNDS; batch *= 2) {
             const int upto = std::min(MAX_ROUNDS, rounds + batch);
             for (; rounds < upto; ++rounds) {
-                TGVG_CK(ctx, cudaMemsetAsync(place, 0xff, sizeof(unsigned) * (2 * wc + 1), st));
-                k_bal_claim<<<lg, 256, 0, st>>>(nl, L, key_slot);
+                k_bal_claim<<<lg, 256, 0, st>>>(nl, L, winner, round_tag(rounds));
                 TGVG_LAUNCHED(ctx);
-                k_bal_accept<<<lg, 256, 0, st>>>(nl, L, key_slot, cell_slot, acc);
-                TGVG_LAUNCHED(ctx);
-                k_bal_again<<<lg, 256, 0, st>>>(nl, h, q, kcell, cell_slot, L, first);
+                k_bal_again<<<lg, 256, 0, st>>>(nl, h, q, kcell, winner, round_tag(rounds), L, first + rounds);
                 TGVG_LAUNCHED(ctx);
             }
             // (at the last round allowed, what lies below the first change is committed)
-            if (rounds == MAX_ROUNDS) {
-                k_bal_limit<<<lg, 256, 0, st>>>(nl, L, first, acc);
-                TGVG_LAUNCHED(ctx);
-            }
+            k_bal_accept<<<lg, 256, 0, st>>>(nl, L, winner, round_tag(rounds - 1), first + rounds - 1,
+                                             rounds == MAX_ROUNDS, acc);
+            TGVG_LAUNCHED(ctx);
             if ((rc = scan_exclusive_async(ctx, acc, nl, apos, asum))) return rc;
-            TGVG_CK(ctx, cudaMemcpyAsync(&change, first, sizeof(change), cudaMemcpyDeviceToHost, st));
+            TGVG_CK(ctx, cudaMemcpyAsync(&change, first + rounds - 1, sizeof(change), cudaMemcpyDeviceToHost, st));
             TGVG_CK(ctx, cudaMemcpyAsync(&na, asum + nsum - 1, sizeof(na), cudaMemcpyDeviceToHost, st));
             TGVG_CK(ctx, cudaStreamSynchronize(st));
             if (change == SLOT_NONE) break;  // settled: the sequential result

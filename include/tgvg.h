@@ -441,7 +441,13 @@ int tgvg_extract_surface_streaming(tgvg_ctx* ctx, const char* balanced_cube_path
                                    float r_root, const char* out_obj_path);
 int tgvg_mesh_size(const tgvg_mesh* m, int64_t* n_verts, int64_t* n_tris, int32_t* has_normals);
 /* Copy out 3 floats per vertex, 3 indices per triangle, 3 floats per normal
- * (any pointer may be null). */
+ * (any pointer may be null).  A context's newest mesh is read from the device,
+ * so a read can fail with TGVG_ERR_CUDA.  The context's next extraction,
+ * tgvg_compute_normals or tgvg_destroy moves it to host memory.  Where the move
+ * fails (TGVG_ERR_NOMEM: no host memory for it), the next extraction or
+ * tgvg_compute_normals fails with that code, and the mesh can be read, or freed
+ * to make room, as before; after tgvg_destroy the mesh is lost and every read
+ * of it returns the code. */
 int tgvg_mesh_read(const tgvg_mesh* m, float* verts, uint32_t* faces, float* normals);
 void tgvg_mesh_free(tgvg_mesh* m);
 /* compute_normals (marching_cubes.hpp:55) over host arrays. */

@@ -169,13 +169,7 @@ enum BufId {
     B_COUNT
 };
 
-// The mesh whose data is in a context's surface output buffers (surface.cu),
-// shared by the context and the mesh; mu orders reads, moves to the host and frees.
-struct tgvg_mesh_link {
-    std::mutex mu;
-    tgvg_mesh* held = nullptr;
-    cudaStream_t stream = nullptr;
-};
+struct tgvg_mesh_link;  // mesh.h
 
 struct tgvg_ctx {
     int device = 0;

@@ -28,36 +28,15 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
-#include <new>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
 #include "fileio.h"
-
-// A mesh stays in the context's own output buffers (B_S_VERTS, B_S_FACES,
-// B_S_NRM, which the context keeps between calls anyway) until something else
-// needs them, so a read is one copy from the device straight into the caller's
-// arrays.  The next extraction, tgvg_compute_normals or tgvg_destroy first moves
-// it to host memory: no more than one mesh per context is on the device, and a
-// mesh can be read at any time, from any thread, also after the context is gone.
-// (Copying every mesh to host vectors and from there to the caller took 16 of
-// the 20 ms of a 1.9 M-cube extraction: zero filling the vectors, page faults
-// and a single-threaded copy of 150 MB; now 0.9 ms.)
-struct tgvg_mesh {
-    int64_t nv = 0, nf = 0;       // vertices, triangles
-    bool has_normals = false;
-    std::shared_ptr<tgvg_mesh_link> link;  // set while the mesh may be on the device
-    const float* d_verts = nullptr;        // 3 per vertex
-    const uint32_t* d_faces = nullptr;     // 3 per triangle
-    const float* d_normals = nullptr;      // 3 per vertex
-    std::unique_ptr<float[]> verts;        // the same in host memory, once moved there
-    std::unique_ptr<uint32_t[]> faces;
-    std::unique_ptr<float[]> normals;
-};
+#include "mesh.h"
 
 // Copies of the mesh on the device to host arrays (null: not wanted).  Called with link->mu held.
-static cudaError_t copy_mesh(const tgvg_mesh* m, float* v, uint32_t* f, float* n) {
+static int copy_mesh(const tgvg_mesh* m, float* v, uint32_t* f, float* n) {
     cudaStream_t st = m->link->stream;
     cudaError_t e = cudaSuccess;
     auto get = [&](void* to, const void* from, size_t bytes) {
@@ -67,34 +46,15 @@ static cudaError_t copy_mesh(const tgvg_mesh* m, float* v, uint32_t* f, float* n
     get(f, m->d_faces, 12ull * m->nf);
     if (m->has_normals) get(n, m->d_normals, 12ull * m->nv);
     const cudaError_t w = cudaStreamSynchronize(st);
-    return e != cudaSuccess ? e : w;
-}
-
-// Moves the mesh that is on the device, if any, to host memory.
-static int mesh_to_host(tgvg_mesh_link* l) {
-    std::lock_guard<std::mutex> lk(l->mu);
-    tgvg_mesh* m = l->held;
-    if (!m) return TGVG_OK;
-    m->verts.reset(new (std::nothrow) float[3 * m->nv + 1]);
-    m->faces.reset(new (std::nothrow) uint32_t[3 * m->nf + 1]);
-    if (m->has_normals) m->normals.reset(new (std::nothrow) float[3 * m->nv + 1]);
-    if (!m->verts || !m->faces || (m->has_normals && !m->normals)) return TGVG_ERR_NOMEM;
-    const cudaError_t e = copy_mesh(m, m->verts.get(), m->faces.get(), m->normals.get());
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return TGVG_ERR_CUDA;
-    }
-    m->d_verts = m->d_normals = nullptr;
-    m->d_faces = nullptr;
-    l->held = nullptr;
-    return TGVG_OK;
+    if (e == cudaSuccess && w == cudaSuccess) return TGVG_OK;
+    cudaGetLastError();
+    return TGVG_ERR_CUDA;
 }
 
 void tgvg_release_mesh(tgvg_ctx* ctx) {
     if (!ctx->mesh_link) return;
-    mesh_to_host(ctx->mesh_link.get());
+    tgvg::mesh_release(ctx->mesh_link.get(), copy_mesh);
     std::lock_guard<std::mutex> lk(ctx->mesh_link->mu);
-    ctx->mesh_link->held = nullptr;
     if (ctx->mesh_link->stream) cudaStreamDestroy(ctx->mesh_link->stream);
     ctx->mesh_link->stream = nullptr;
 }
@@ -712,7 +672,7 @@ static int mesh_buffers(tgvg_ctx* ctx) {
         TGVG_CK(ctx, cudaStreamCreateWithFlags(&l->stream, cudaStreamNonBlocking));
         ctx->mesh_link = std::move(l);
     }
-    const int rc = mesh_to_host(ctx->mesh_link.get());
+    const int rc = mesh_to_host(ctx->mesh_link.get(), copy_mesh);
     return rc ? ctx->fail(rc, "moving the previous mesh to host memory") : TGVG_OK;
 }
 
@@ -791,19 +751,7 @@ extern "C" int tgvg_mesh_size(const tgvg_mesh* m, int64_t* nv, int64_t* nf, int3
 
 extern "C" int tgvg_mesh_read(const tgvg_mesh* m, float* verts, uint32_t* faces, float* normals) {
     if (!m) return TGVG_ERR_INVALID;
-    if (m->link) {
-        std::lock_guard<std::mutex> lk(m->link->mu);
-        if (m->link->held == m) {
-            if (copy_mesh(m, verts, faces, normals) == cudaSuccess) return TGVG_OK;
-            cudaGetLastError();
-            return TGVG_ERR_CUDA;
-        }
-    }
-    if (m->nv > 0 && !m->verts) return TGVG_ERR_NOMEM;  // there was no host memory for it when its context went
-    if (verts && m->verts) std::memcpy(verts, m->verts.get(), 12ull * m->nv);
-    if (faces && m->faces) std::memcpy(faces, m->faces.get(), 12ull * m->nf);
-    if (normals && m->normals) std::memcpy(normals, m->normals.get(), 12ull * m->nv);
-    return TGVG_OK;
+    return tgvg::mesh_read(m, verts, faces, normals, copy_mesh);
 }
 
 extern "C" void tgvg_mesh_free(tgvg_mesh* m) {

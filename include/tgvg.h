@@ -357,11 +357,18 @@ int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, int64_t n, f
 /* Warm-start u of n cubes: features, forward pass and the median indicator
  * (FP32, reference order) added, all on the device.  Host arrays in and out;
  * the _dev form takes device cubes / histograms / u and host leaves, and
- * leaves u on the context stream for tgvg_tgv_minimize_dev. */
+ * leaves u on the context stream for tgvg_tgv_minimize_dev.  Waits inside the
+ * network's kernel are bounded (under a second): when one runs out, the calls
+ * that wait for their result (tgvg_mlp_predict, tgvg_mlp_warm_start) return
+ * TGVG_ERR_TIMEOUT; the _dev form, which does not wait, leaves NaN in u, and
+ * the context's next solve returns TGVG_ERR_TIMEOUT, once, before it starts. */
 int tgvg_mlp_warm_start(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* cubes, const uint32_t* hists, int64_t n,
                         int32_t nbins, const tgvg_leaf* leaves, int32_t nleaf, float* u);
 int tgvg_mlp_warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_cubes, const uint32_t* d_hists,
                             int64_t n, int32_t nbins, const tgvg_leaf* leaves, int32_t nleaf, float* d_u);
+/* Polls (of up to 20 us) after which such a wait gives up: 0 = at once, for tests
+ * of the error path; values above the default of 32768 are taken as that. */
+int tgvg_mlp_set_wait_limit(tgvg_mlp* m, int32_t polls);
 /* Gradient of the mean squared error over all n rows (for checks; host arrays). */
 int tgvg_mlp_grad(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, const float* t, int64_t n, float* grad,
                   float* loss);

@@ -156,6 +156,7 @@ _SIGS = {
     "tgvg_mlp_predict": ([P, P, P, C.c_int64, P], C.c_int),
     "tgvg_mlp_warm_start": ([P, P, P, P, C.c_int64, C.c_int32, P, C.c_int32, P], C.c_int),
     "tgvg_mlp_warm_start_dev": ([P, P, P, P, C.c_int64, C.c_int32, P, C.c_int32, P], C.c_int),
+    "tgvg_mlp_set_wait_limit": ([P, C.c_int32], C.c_int),
     "tgvg_mlp_grad": ([P, P, P, P, C.c_int64, P, P], C.c_int),
     "tgvg_mlp_train": ([P, P, P, P, C.c_int64, C.c_int32, C.c_int32, C.c_float, C.c_uint64, P], C.c_int),
     "tgvg_build_cubes": ([P, P, P, C.c_float, P, C.c_int64, C.POINTER(C.c_int64)], C.c_int),

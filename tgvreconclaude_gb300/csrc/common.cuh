@@ -152,7 +152,7 @@ enum BufId {
     B_Q1, B_DAT, B_SNAP, B_LID, B_LEAVES, B_ACC, B_FLAGS, B_RANGES, B_RESID, B_LVSTAT,
     B_BARB, B_P4B, B_Q4B, B_Q1B, B_FSLOT, B_FHALO, B_FHCNT,
     // learned warm start
-    B_M_X, B_M_T, B_M_IDX, B_M_Y, B_M_LEAVES, B_M_LEAFID, B_M_BOXES,
+    B_M_X, B_M_T, B_M_IDX, B_M_Y, B_M_LEAVES, B_M_LEAFID, B_M_BOXES, B_M_ERR,
     // surface extraction
     B_S_CUBES, B_S_STATE, B_S_KEYS, B_S_DEPTH, B_S_U, B_S_HD, B_S_HKEYS, B_S_HMIN, B_S_HMAX, B_S_NBR,
     B_S_FLAGS, B_S_QIDX, B_S_SCAN, B_S_RANK, B_S_LEAF, B_S_QKEY, B_S_QPOS, B_S_QFLIP, B_S_VTK, B_S_VTF,
@@ -209,6 +209,7 @@ struct tgvg_ctx {
     bool capturing = false;            // the level loop is being captured
     size_t device_budget = 0;          // solve footprint above which the state lives in host memory (0: never)
     bool paged_now = false;            // the running solve's state lives in host memory (no TMA-staged schedule)
+    bool mlp_pending = false;          // a warm start that nobody waited for has run since the last mlp_take_error
     std::shared_ptr<tgvg_mesh_link> mesh_link;  // set by the first surface extraction
     tgvg_ctx() {
         for (auto& m : tune)
@@ -274,5 +275,8 @@ int pyramid_dims(int32_t w, int32_t h, int32_t* dims);
 int scan_exclusive(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, int64_t* total);
 int64_t scan_sums_len(int64_t n);
 int scan_tile_sums(tgvg_ctx* ctx, int* sums, int nt);
+// TGVG_ERR_TIMEOUT, once, when a wait of an earlier tgvg_mlp_warm_start_dev ran out; waits for the stream
+// only where one was called (mlp.cu).
+int mlp_take_error(tgvg_ctx* ctx);
 int scan_exclusive_async(tgvg_ctx* ctx, const int* d_in, int64_t n, int* d_out, int* sums);
 }  // namespace tgvg

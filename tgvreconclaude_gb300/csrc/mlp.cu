@@ -341,8 +341,10 @@ __device__ __forceinline__ uint32_t pack_top(float a, float b) {
 // eight tiles in flight cover one another's waits (the 64 registers of 1024
 // threads and the 512 TMEM columns both end at eight).  A group's tiles are
 // neighbours: the next tile's rows are fetched into L2 ahead, and its chunk is
-// looked up again only where one ends.  The waits are bounded; a group that gives
-// up issues no more products, sets *err and yields NaN.
+// looked up again only where one ends.  The waits are bounded; a warp that gives
+// up touches neither its operands nor TMEM again, sets *err and yields NaN, and a
+// group whose products' warp gave up issues no more and waits, again bounded, for
+// the ones in flight before the TMEM goes.
 //
 // Bytes: 16 + 4 NB read and 4 written per cube, 19 us for 2.2 M cubes of 10 bins;
 // what bounds it is the instructions of a row's features and its two epilogues
@@ -382,8 +384,9 @@ __device__ __forceinline__ void tc_product(uint32_t d, uint32_t a_at, uint32_t b
     }
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
-__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
-    for (int spin = 0; spin < (1 << 15); ++spin) {  // at most 20 us each
+constexpr int TC_POLLS = 1 << 15;  // of a wait, at most 20 us each
+__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity, int polls) {
+    for (int spin = 0; spin < polls; ++spin) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\t"
@@ -433,7 +436,7 @@ template <int NB, int SRC>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, const uint32_t* __restrict__ hists,
           const LeafBox* __restrict__ boxes, int nleaf, const int* __restrict__ leaf_id,
-          const __nv_bfloat16* __restrict__ weights, float* __restrict__ out, int* __restrict__ err) {
+          const __nv_bfloat16* __restrict__ weights, float* __restrict__ out, int* __restrict__ err, int polls) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ FeatureTables tab;
     __shared__ __align__(8) unsigned long long s_bar[TC_GROUPS];
@@ -462,8 +465,12 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
     const uint32_t d = s_tmem + group * 64;                          // the group's columns
     const uint32_t mine = d + ((uint32_t)(warp & 3) * 32u << 16);  // this warp's lanes of them
     const bool vec = SRC && bins_aligned<NB>(hists);
-    uint32_t phase = 0;
-    bool ok = true;
+    uint32_t phase = 0;  // of the products waited for next
+    bool ok = true;      // the same for all of a warp
+    auto wait = [&] {
+        if (ok) ok = __all_sync(0xffffffffu, tc_wait(bar, phase & 1, polls));
+        if (ok) ++phase;
+    };
     // Each group's tiles are neighbours, so its chunk seldom changes.
     const int64_t tiles = ((int64_t)n + 127) / 128, runs = (int64_t)gridDim.x * TC_GROUPS,
                   run = blockIdx.x + (int64_t)group * gridDim.x;
@@ -508,23 +515,25 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
             }
         }
         // layer 1: columns 48..63 hold the features, 64..79 the ones
-        *reinterpret_cast<uint4*>(A + 6 * TC_CORE + row * 16) = lo;
-        *reinterpret_cast<uint4*>(A + 7 * TC_CORE + row * 16) = hi;
+        if (ok) {
+            *reinterpret_cast<uint4*>(A + 6 * TC_CORE + row * 16) = lo;
+            *reinterpret_cast<uint4*>(A + 7 * TC_CORE + row * 16) = hi;
+        }
         tc_group_sync(group);
         if (row == 0 && ok) tc_product(d, a_at + 6 * TC_CORE, w_at + TC_B1, 64, 2, bar);
         for (int layer = 0; layer < 2; ++layer) {
-            ok = ok && tc_wait(bar, phase & 1);
-            ++phase;
-            __syncwarp();
+            wait();
+            if (ok) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t r[32];
-                tc_load32(mine + half * 32, r);
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t r[32];
+                    tc_load32(mine + half * 32, r);
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(A + (half * 4 + c) * TC_CORE + row * 16) =
-                        make_uint4(relu_pack(r[8 * c], r[8 * c + 1]), relu_pack(r[8 * c + 2], r[8 * c + 3]),
-                                   relu_pack(r[8 * c + 4], r[8 * c + 5]), relu_pack(r[8 * c + 6], r[8 * c + 7]));
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(A + (half * 4 + c) * TC_CORE + row * 16) =
+                            make_uint4(relu_pack(r[8 * c], r[8 * c + 1]), relu_pack(r[8 * c + 2], r[8 * c + 3]),
+                                       relu_pack(r[8 * c + 4], r[8 * c + 5]), relu_pack(r[8 * c + 6], r[8 * c + 7]));
+                }
             }
             tc_group_sync(group);
             if (row == 0 && ok) {
@@ -532,18 +541,17 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
                 else tc_product(d, a_at, w_at + TC_B3, 16, 5, bar);
             }
         }
-        ok = ok && tc_wait(bar, phase & 1);
-        ++phase;
-        __syncwarp();
-        uint32_t y;
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;"
-                     : "=r"(y) : "r"(mine) : "memory");
-        if (i < n) {
-            const float v = ok ? __uint_as_float(y) : __int_as_float(0x7fc00000);
-            out[i] = SRC ? fadd(med, v) : v;
-        }
+        wait();
+        uint32_t y = 0x7fc00000u;
+        if (ok)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;"
+                         : "=r"(y) : "r"(mine) : "memory");
+        if (i < n) out[i] = SRC ? fadd(med, __uint_as_float(y)) : __uint_as_float(y);
     }
-    if (!ok) atomicOr(err, 1);
+    if (!ok) {
+        if (lane == 0) atomicOr(err, 1);
+        if (row == 0) tc_wait(bar, phase & 1, TC_POLLS);  // the products still in flight
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -554,13 +562,14 @@ k_forward(int n, const uint4* __restrict__ X, const uint4* __restrict__ cubes, c
 // One inference launch; d_id null with leaves means ascending chunks.
 template <int NB, int SRC>
 static int launch_forward(tgvg_ctx* ctx, int64_t n, const uint32_t* X, const tgvg_cube* d_c, const uint32_t* d_h,
-                          const LeafBox* boxes, int nleaf, const int* d_id, const __nv_bfloat16* tc, float* out, int* err) {
+                          const LeafBox* boxes, int nleaf, const int* d_id, const __nv_bfloat16* tc, float* out, int* err,
+                          int polls) {
     TGVG_CK(ctx, cudaFuncSetAttribute(k_forward<NB, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     const int64_t tiles = (n + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->sm_count);  // a few tiles spread over the SMs
     k_forward<NB, SRC><<<grid, TC_THREADS, TC_SMEM, ctx->stream>>>(
         (int)n, reinterpret_cast<const uint4*>(X), reinterpret_cast<const uint4*>(d_c), d_h, boxes, nleaf, d_id, tc, out,
-        err);
+        err, polls);
     TGVG_LAUNCHED(ctx);
     return TGVG_OK;
 }
@@ -908,8 +917,8 @@ struct tgvg_mlp {
     float* d_loss = nullptr;
     uint32_t* d_frag = nullptr;
     __nv_bfloat16* d_tc = nullptr;
-    int* d_err = nullptr;  // set by an inference wait that ran out
     int step = 0;
+    int polls = TC_POLLS;  // of an inference wait
 };
 
 static int mlp_repack(tgvg_ctx* ctx, tgvg_mlp* m) {
@@ -928,7 +937,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
         if (cudaMalloc(b, sizeof(float) * P_N) != cudaSuccess) { delete m; return TGVG_ERR_NOMEM; }
     if (cudaMalloc(&m->d_loss, sizeof(float)) != cudaSuccess ||
         cudaMalloc(&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess ||
-        cudaMalloc(&m->d_tc, TC_W) != cudaSuccess || cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&m->d_tc, TC_W) != cudaSuccess) {
         delete m;
         return TGVG_ERR_NOMEM;
     }
@@ -944,7 +953,6 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
     for (int k = 0; k < 64 * 64; ++k) p[P_W2 + k] = u2(rng);
     for (int k = 0; k < 64; ++k) p[P_W3 + k] = u3(rng);
     TGVG_CK(ctx, cudaMemcpyAsync(m->d_prm, p.data(), sizeof(float) * P_N, cudaMemcpyHostToDevice, ctx->stream));
-    TGVG_CK(ctx, cudaMemsetAsync(m->d_err, 0, sizeof(int), ctx->stream));
     TGVG_CK(ctx, cudaMemsetAsync(m->d_m1, 0, sizeof(float) * P_N, ctx->stream));
     TGVG_CK(ctx, cudaMemsetAsync(m->d_m2, 0, sizeof(float) * P_N, ctx->stream));
     int rc = mlp_repack(ctx, m);
@@ -957,7 +965,7 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
 extern "C" int tgvg_mlp_destroy(tgvg_mlp* m) {
     if (!m) return TGVG_ERR_INVALID;
     cudaFree(m->d_prm); cudaFree(m->d_m1); cudaFree(m->d_m2); cudaFree(m->d_grad); cudaFree(m->d_wr);
-    cudaFree(m->d_loss); cudaFree(m->d_frag); cudaFree(m->d_tc); cudaFree(m->d_err);
+    cudaFree(m->d_loss); cudaFree(m->d_frag); cudaFree(m->d_tc);
     delete m;
     return TGVG_OK;
 }
@@ -1011,14 +1019,38 @@ extern "C" int tgvg_mlp_features(tgvg_ctx* ctx, const tgvg_cube* cubes, const ui
     return TGVG_OK;
 }
 
-// Waits for the stream and reports an inference whose wait ran out.
-static int inference_done(tgvg_ctx* ctx, tgvg_mlp* m) {
+// Set by inference waits that run out: [0] in a call that waits for its result,
+// [1] in tgvg_mlp_warm_start_dev, which does not (mlp_take_error).  Null: no memory.
+static int* inference_error(tgvg_ctx* ctx) {
+    const bool fresh = !ctx->bufs[B_M_ERR].p;
+    int* e = (int*)ctx->buf(B_M_ERR, 2 * sizeof(int));
+    if (e && fresh && cudaMemsetAsync(e, 0, 2 * sizeof(int), ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return e;
+}
+
+// Waits for the stream; reports the calling inference when a wait of it ran out.
+static int inference_done(tgvg_ctx* ctx, int* err) {
     int e = 0;
-    TGVG_CK(ctx, cudaMemcpyAsync(&e, m->d_err, sizeof(e), cudaMemcpyDeviceToHost, ctx->stream));
+    TGVG_CK(ctx, cudaMemcpyAsync(&e, err, sizeof(e), cudaMemcpyDeviceToHost, ctx->stream));
     TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
     if (!e) return TGVG_OK;
-    TGVG_CK(ctx, cudaMemsetAsync(m->d_err, 0, sizeof(int), ctx->stream));
+    TGVG_CK(ctx, cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
     return ctx->fail(TGVG_ERR_TIMEOUT, "a tensor-core wait of the network timed out");
+}
+
+int tgvg::mlp_take_error(tgvg_ctx* ctx) {
+    if (!ctx->mlp_pending) return TGVG_OK;
+    ctx->mlp_pending = false;
+    return inference_done(ctx, (int*)ctx->bufs[B_M_ERR].p + 1);
+}
+
+extern "C" int tgvg_mlp_set_wait_limit(tgvg_mlp* m, int32_t polls) {
+    if (!m || polls < 0) return TGVG_ERR_INVALID;
+    m->polls = polls < TC_POLLS ? polls : TC_POLLS;
+    return TGVG_OK;
 }
 
 extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, int64_t n, float* y) {
@@ -1027,18 +1059,19 @@ extern "C" int tgvg_mlp_predict(tgvg_ctx* ctx, tgvg_mlp* m, const uint16_t* X, i
     if (n == 0) return TGVG_OK;
     auto* d_x = (uint32_t*)ctx->buf(B_M_X, sizeof(uint32_t) * 8 * n);
     auto* d_y = (float*)ctx->buf(B_M_Y, sizeof(float) * n);
-    if (!d_x || !d_y) return TGVG_ERR_NOMEM;
+    int* err = inference_error(ctx);
+    if (!d_x || !d_y || !err) return TGVG_ERR_NOMEM;
     TGVG_CK(ctx, cudaMemcpyAsync(d_x, X, sizeof(uint32_t) * 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-    int rc = launch_forward<8, 0>(ctx, n, d_x, nullptr, nullptr, nullptr, 0, nullptr, m->d_tc, d_y, m->d_err);
+    int rc = launch_forward<8, 0>(ctx, n, d_x, nullptr, nullptr, nullptr, 0, nullptr, m->d_tc, d_y, err, m->polls);
     if (rc) return rc;
     TGVG_CK(ctx, cudaMemcpyAsync(y, d_y, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    return inference_done(ctx, m);
+    return inference_done(ctx, err);
 }
 
 // Warm-start u on the device (u = median + network).  Device cubes / histograms
 // / output, host leaves.  Called with ctx->mu held.
 static int warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_c, const uint32_t* d_h, int64_t n,
-                          int32_t nbins, const tgvg_leaf* leaves, int32_t nleaf, float* d_u) {
+                          int32_t nbins, const tgvg_leaf* leaves, int32_t nleaf, float* d_u, int* err) {
     auto* d_b = (LeafBox*)ctx->buf(B_M_BOXES, sizeof(LeafBox) * std::max(1, nleaf));
     if (!d_b) return TGVG_ERR_NOMEM;
     // Ranges that ascend without overlap (a treetop's) are found by bisection;
@@ -1061,10 +1094,10 @@ static int warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_c, cons
         TGVG_LAUNCHED(ctx);
     }
     if (nbins == 8)
-        return sorted ? launch_forward<8, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, m->d_err)
-                      : launch_forward<8, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, m->d_err);
-    return sorted ? launch_forward<10, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, m->d_err)
-                  : launch_forward<10, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, m->d_err);
+        return sorted ? launch_forward<8, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, err, m->polls)
+                      : launch_forward<8, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, err, m->polls);
+    return sorted ? launch_forward<10, 1>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, nullptr, m->d_tc, d_u, err, m->polls)
+                  : launch_forward<10, 2>(ctx, n, nullptr, d_c, d_h, d_b, nleaf, d_id, m->d_tc, d_u, err, m->polls);
 }
 
 static bool warm_start_args_ok(tgvg_ctx* ctx, tgvg_mlp* m, const void* c, const void* h, int64_t n, int32_t nbins,
@@ -1081,13 +1114,14 @@ extern "C" int tgvg_mlp_warm_start(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* 
     auto* d_c = (tgvg_cube*)ctx->buf(B_T_CUBES, sizeof(tgvg_cube) * n);
     auto* d_h = (uint32_t*)ctx->buf(B_T_HISTS, sizeof(uint32_t) * nbins * n);
     auto* d_u = (float*)ctx->buf(B_M_Y, sizeof(float) * n);
-    if (!d_c || !d_h || !d_u) return TGVG_ERR_NOMEM;
+    int* err = inference_error(ctx);
+    if (!d_c || !d_h || !d_u || !err) return TGVG_ERR_NOMEM;
     TGVG_CK(ctx, cudaMemcpyAsync(d_c, cubes, sizeof(tgvg_cube) * n, cudaMemcpyHostToDevice, ctx->stream));
     TGVG_CK(ctx, cudaMemcpyAsync(d_h, hists, sizeof(uint32_t) * nbins * n, cudaMemcpyHostToDevice, ctx->stream));
-    int rc = warm_start_dev(ctx, m, d_c, d_h, n, nbins, leaves, nleaf, d_u);
+    int rc = warm_start_dev(ctx, m, d_c, d_h, n, nbins, leaves, nleaf, d_u, err);
     if (rc) return rc;
     TGVG_CK(ctx, cudaMemcpyAsync(u, d_u, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    return inference_done(ctx, m);
+    return inference_done(ctx, err);
 }
 
 extern "C" int tgvg_mlp_warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cube* d_cubes,
@@ -1096,7 +1130,10 @@ extern "C" int tgvg_mlp_warm_start_dev(tgvg_ctx* ctx, tgvg_mlp* m, const tgvg_cu
     if (!warm_start_args_ok(ctx, m, d_cubes, d_hists, n, nbins, leaves, nleaf, d_u)) return TGVG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (n == 0) return TGVG_OK;
-    return warm_start_dev(ctx, m, d_cubes, d_hists, n, nbins, leaves, nleaf, d_u);
+    int* err = inference_error(ctx);
+    if (!err) return TGVG_ERR_NOMEM;
+    ctx->mlp_pending = true;
+    return warm_start_dev(ctx, m, d_cubes, d_hists, n, nbins, leaves, nleaf, d_u, err + 1);
 }
 
 // Gradient of the mean squared error of the whole set (one batch), for checks.

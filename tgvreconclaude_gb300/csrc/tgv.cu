@@ -3509,6 +3509,7 @@ int tgv_solve_dev(tgvg_ctx* ctx, const tgvg_cube* d_cubes, const uint32_t* d_his
     k_hash_insert<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(n, keys, hv);
     TGVG_LAUNCHED(ctx);
     TGVG_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (const int rc = mlp_take_error(ctx)) return rc;  // the initial u may be that warm start
     if (h_flags[1]) return ctx->fail(TGVG_ERR_INVALID, "cube depth outside 0..21");
     if (mode == M_STREAM && h_flags[0])
         return ctx->fail(TGVG_ERR_UNSORTED, "streaming semantics need Morton-sorted cubes");

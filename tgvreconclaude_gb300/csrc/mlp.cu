@@ -59,8 +59,8 @@ __device__ __forceinline__ void mma_bf16(float& d0, float& d1, float& d2, float&
 }
 
 // An FP32 value as the exact sum of three bf16 parts (8 significant bits each,
-// cut off, not rounded, so nothing overflows); a non-finite value stays whole
-// in the first part.
+// cut off, not rounded, so nothing overflows); the first part alone holds an
+// infinity, or a NaN as arithmetic makes them (payload in the upper half).
 __device__ __forceinline__ void split_bf16(float v, float& hi, float& mid, float& lo) {
     hi = __uint_as_float(__float_as_uint(v) & 0xffff0000u);
     const float r = isfinite(v) ? v - hi : 0.f;
@@ -79,7 +79,9 @@ __device__ __forceinline__ __nv_bfloat16 tc_weight(const float* __restrict__ prm
     if (k >= width + 3 || (l3 && j > 0)) return __float2bfloat16_rn(0.f);
     if (k < width) return __float2bfloat16_rn(prm[l3 ? P_W3 + k : (l1 ? P_W1 : P_W2) + k * MLP_H + j]);
     float p[3];
-    split_bf16(prm[(l3 ? P_B3 : (l1 ? P_B1 : P_B2)) + j], p[0], p[1], p[2]);
+    const float b = prm[(l3 ? P_B3 : (l1 ? P_B1 : P_B2)) + j];
+    split_bf16(b, p[0], p[1], p[2]);
+    if (isnan(b)) p[0] = b;  // cut off, a payload in the low half would leave an infinity
     return __float2bfloat16_rn(p[k - width]);  // exact: a bf16 value
 }
 

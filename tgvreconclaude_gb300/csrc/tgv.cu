@@ -896,9 +896,11 @@ __device__ __forceinline__ bool grid_sync(unsigned* count, unsigned* gen, int* e
 template <int MODE>
 __host__ __device__ __forceinline__ int unit_slots(int nslot) { return MODE == M_STREAM ? nslot : 1; }
 
-// Stopping test of the unit's slots, run by block 0 between barriers (k_check's logic).
+// Stopping test of the unit's slots, run by block 0 between barriers (k_check's
+// logic); whether one of this thread's slots goes on.
 template <int MODE>
-__device__ __forceinline__ void check_slots(const IterArgs& a, int it) {
+__device__ __forceinline__ bool check_slots(const IterArgs& a, int it) {
+    bool left = false;
     for (int s = a.slot0 + threadIdx.x; s < a.slot0 + unit_slots<MODE>(a.nslot); s += blockDim.x) {
         if (a.done[s]) continue;
         double* q = a.acc + s * 4;
@@ -907,8 +909,10 @@ __device__ __forceinline__ void check_slots(const IterArgs& a, int it) {
         const double rel = den > 0.0 ? num / den : 0.0;
         a.resid[s] = rel;
         if (rel <= (double)a.tol) { a.done[s] = 1; a.iters_run[s] = it + 1; }
+        else left = true;
         q[0] = q[1] = q[2] = q[3] = 0.0;
     }
+    return left;
 }
 
 // Every iteration of one level in ONE cooperative launch (levels small enough
@@ -1381,6 +1385,14 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, unsigned rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
     return out;
 }
+__device__ __forceinline__ unsigned cluster_ctas() {
+    unsigned n;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 template <bool ONE>
 __device__ __forceinline__ float4 ld_record(uint32_t addr) {
     float4 r;
@@ -1407,7 +1419,7 @@ __device__ __forceinline__ float4 face_record(int k, const float4& A, const floa
 template <int MODE, bool STOP, bool ONE>
 __global__ void __launch_bounds__(REG_CTA_MAX) k_level_reg(IterArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_ng;
+    __shared__ int s_ng, s_left;  // s_left: some leaf goes on (streaming semantics)
     const int chunk = a.chunk, x = threadIdx.x, lane = x & 31;
     const unsigned me = ONE ? 0u : cluster_rank();
     float4* s_bar = reinterpret_cast<float4*>(smem_raw);
@@ -1493,9 +1505,17 @@ __global__ void __launch_bounds__(REG_CTA_MAX) k_level_reg(IterArgs a) {
             w.add(work ? slot : -1, dp, np, a.acc, 0, lane);
             w.flush(a.acc, 0, lane);
             level_barrier<ONE>();
-            if (me == 0) check_slots<MODE>(a, it);
+            if (me == 0) {
+                const bool left = check_slots<MODE>(a, it);
+                if (MODE == M_STREAM) {  // told to every CTA
+                    const int any = __syncthreads_or(left);
+                    const uint32_t to = (uint32_t)__cvta_generic_to_shared(&s_left);
+                    if (ONE) { if (x == 0) s_left = any; }
+                    else if (x < (int)cluster_ctas()) st_cluster(cluster_addr(to, x), any);
+                }
+            }
             level_barrier<ONE>();
-            if (MODE != M_STREAM && __ldcg(a.done + a.slot0)) break;  // the same for every thread
+            if (MODE == M_STREAM ? !s_left : __ldcg(a.done + a.slot0) != 0) break;  // the same for every thread
             if (work) work = __ldcg(a.done + slot) == 0;
         } else {
             level_barrier<ONE>();
@@ -1530,7 +1550,7 @@ constexpr int GRID_K2_THREADS = 832;  // threads of a block at two cubes per thr
 struct GridArgs {
     float4* gx;      // [4][n] bars and face records of cubes that other blocks read, then staged records
     int* pub;        // [n] which of them: bit 0 bars, bit 1 + k face record k
-    unsigned* flag;  // the barrier's counter
+    unsigned* flag;  // the barrier's counter; then whether every leaf has stopped (streaming semantics)
     int gcap;        // staged records with room in shared memory
 };
 
@@ -1694,11 +1714,14 @@ __global__ void __launch_bounds__(K == 1 ? REG_CTA_MAX : GRID_K2_THREADS, 1) k_l
         if (STOP && res) {
             wp.flush(a.acc, 0, lane);
             if (!flag_barrier(g.flag, ++epoch, a.err)) return;
-            if (blockIdx.x == 0) check_slots<MODE>(a, it);
+            if (blockIdx.x == 0) {
+                const bool left = check_slots<MODE>(a, it);
+                if (MODE == M_STREAM && !__syncthreads_or(left) && x == 0) __stcg(g.flag + 1, 1u);
+            }
         }
         if (!flag_barrier(g.flag, ++epoch, a.err)) return;
         if (STOP && res) {
-            if (MODE != M_STREAM && __ldcg(a.done + a.slot0)) break;  // the same for every block
+            if (MODE == M_STREAM ? __ldcg(g.flag + 1) != 0 : __ldcg(a.done + a.slot0) != 0) break;  // the same for every block
 #pragma unroll
             for (int k = 0; k < K; ++k)
                 if (work[k]) work[k] = __ldcg(a.done + slot[k]) == 0;
@@ -2797,9 +2820,9 @@ static int grid_capacity(tgvg_ctx* ctx, int n, int* out) {
     }
     *out = c;
     if (c > 0 && n <= chip_max(ctx, c) && grid_launch(n, c).k == 0) {
-        if (!ctx->buf(B_R_PUB, 4ull * (n + 1))) return TGVG_ERR_NOMEM;
+        if (!ctx->buf(B_R_PUB, 4ull * (n + 2))) return TGVG_ERR_NOMEM;
     } else if (grid_launch(n, c).k > 0) {
-        if (!ctx->buf(B_R_GX, 160ull * n) || !ctx->buf(B_R_PUB, 4ull * (n + 1))) return TGVG_ERR_NOMEM;
+        if (!ctx->buf(B_R_GX, 160ull * n) || !ctx->buf(B_R_PUB, 4ull * (n + 2))) return TGVG_ERR_NOMEM;
     }
     return TGVG_OK;
 }
@@ -2970,12 +2993,12 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
             ChipArgs g;
             const int grid = CHIP_BLOCKS * ctx->sm_count;
             g.rc = (a.n + grid - 1) / grid;
-            g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 1));
+            g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 2));
             if (!g.pub) return TGVG_ERR_NOMEM;
             g.flag = (unsigned*)(g.pub + a.n);
             a.it0 = it0;
             a.iters = count;
-            TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 1), ctx->stream));
+            TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 2), ctx->stream));
             void* args[] = {&a, &g};
             const cudaError_t e = cudaLaunchCooperativeKernel(chip_kernel<MODE>(stop), dim3(grid), dim3(CHIP_THREADS),
                                                               args, ctx->chip_smem, ctx->stream);
@@ -2985,14 +3008,14 @@ static int run_segment(tgvg_ctx* ctx, IterArgs a, int cfg, int it0, int count, b
         }
         GridArgs g;
         g.gx = (float4*)ctx->buf(B_R_GX, 160ull * a.n);
-        g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 1));
+        g.pub = (int*)ctx->buf(B_R_PUB, 4ull * (a.n + 2));
         if (!g.gx || !g.pub) return TGVG_ERR_NOMEM;
         g.flag = (unsigned*)(g.pub + a.n);
         const size_t fixed = grid_bytes(l);
         g.gcap = std::min(6 * l.k * l.threads, (int)((ctx->grid_smem - fixed) / 16));
         a.it0 = it0;
         a.iters = count;
-        TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 1), ctx->stream));
+        TGVG_CK(ctx, cudaMemsetAsync(g.pub, 0, 4ull * (a.n + 2), ctx->stream));
         void* args[] = {&a, &g};
         const cudaError_t e = cudaLaunchCooperativeKernel(grid_kernel<MODE>(l.k, stop), dim3(l.blocks), dim3(l.threads),
                                                           args, fixed + 16 * (size_t)g.gcap, ctx->stream);

@@ -180,7 +180,8 @@ extern "C" int tgvg_set_schedule(tgvg_ctx* ctx, int32_t mode, int32_t cls, int32
     if (!ctx || mode < 0 || mode > 2 || cls < -1 || cls > 31 || cfg < -1 || cfg > 24) return TGVG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
     for (int c = 0; c < 32; ++c)
-        if (cls < 0 || c == cls) ctx->tune[mode][c] = cfg;
+        if (cls < 0 || c == cls)
+            for (int& k : ctx->tune[mode][c]) k = cfg;
     return TGVG_OK;
 }
 

@@ -171,6 +171,9 @@ enum BufId {
 
 struct tgvg_mesh_link;  // mesh.h
 
+// One cluster of up to 8 CTAs, one of 16, registers of the whole GPU, its shared memory, none (tune_kind, tgv.cu).
+constexpr int TUNE_KINDS = 5;
+
 struct tgvg_ctx {
     int device = 0;
     int sm_count = 0;
@@ -184,7 +187,8 @@ struct tgvg_ctx {
     cudaEvent_t ev[4] = {};
     bool timing = false;               // per-launch events on the largest level
     std::vector<cudaEvent_t> tev;      // pool for those events
-    int tune[3][32];                   // chosen iteration schedule per mode and log2(size) class, -1 = untuned
+    // chosen iteration schedule per mode, log2(size) class and on-chip kernel that holds the unit, -1 = untuned
+    int tune[3][32][TUNE_KINDS];
     int coop_max[3][2] = {};           // co-resident blocks of the persistent kernel per mode / stop
     int cluster_max[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};  // usable cluster size per mode / stop (-1 unknown)
     int iter_occ[3][2][2] = {};        // blocks/SM of the sweep kernels [mode][register-capped][dual, primal]
@@ -213,7 +217,8 @@ struct tgvg_ctx {
     std::shared_ptr<tgvg_mesh_link> mesh_link;  // set by the first surface extraction
     tgvg_ctx() {
         for (auto& m : tune)
-            for (int& c : m) c = -1;
+            for (auto& c : m)
+                for (int& k : c) k = -1;
     }
 
     // Device buffer `id` with room for `bytes` (grow-only; contents are not kept

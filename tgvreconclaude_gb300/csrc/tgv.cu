@@ -2819,6 +2819,7 @@ static int grid_capacity(tgvg_ctx* ctx, int n, int* out) {
         cudaGetLastError();
     }
     *out = c;
+    if (n == 0) return TGVG_OK;  // only asked for
     if (c > 0 && n <= chip_max(ctx, c) && grid_launch(n, c).k == 0) {
         if (!ctx->buf(B_R_PUB, 4ull * (n + 2))) return TGVG_ERR_NOMEM;
     } else if (grid_launch(n, c).k > 0) {
@@ -3109,10 +3110,26 @@ static int tune_candidates(tgvg_ctx* ctx, int n, std::vector<int>& cands) {
 // whole GPU): over 16 iterations that made 3.7 us look like 5.
 static int trial_iters(int cfg) { return cfg == CFG_SMEM || cfg == CFG_REG ? 4 * TUNE_SEG : TUNE_SEG; }
 
+// The entry of the schedule table for a unit of n cubes.  The on-chip kernels'
+// limits lie inside the size classes (2,048 in that of 2,048 to 4,095; on 152 SMs
+// 252,928 and about 541,000), and a unit beyond a limit has other candidates and
+// other times than one within it, so a pick applies only to units that the same
+// kernel holds.  (With one pick a class, what a unit of 530,000 cubes ran with
+// depended on whether one of 600,000 had been solved before it.)
+template <int MODE>
+static int tune_entry(tgvg_ctx* ctx, int n, int** pick) {
+    int rc, rs = 0, gb = 0;
+    if ((rc = reg_capacity<MODE>(ctx, &rs)) || (rc = grid_capacity<MODE>(ctx, 0, &gb))) return rc;
+    const int kind = n <= SMEM_MAX_N && rs > 0 ? 0 : n <= rs * REG_CTA_MAX ? 1 : grid_launch(n, gb).k > 0 ? 2
+                   : n <= chip_max(ctx, gb) ? 3 : TUNE_KINDS - 1;
+    *pick = &ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, n))][kind];
+    return TGVG_OK;
+}
+
 // The schedule a unit of n cubes runs with, or -1 when the online autotuner
 // will first time the candidates on it.  The schedule for the unit's size
-// class (floor(log2 n)) is taken from the context's table; the first time a
-// class is met in a fixed-count solve with enough iterations, its first
+// class (floor(log2 n)) is taken from the context's table (tune_entry); the first
+// time an entry is met in a fixed-count solve with enough iterations, its first
 // segments try each candidate (trial_iters) and keep the fastest per iteration
 // (the tried iterations count toward the solve).  Also makes sure the
 // occupancy figures the launches need are cached.
@@ -3121,7 +3138,9 @@ static int plan_schedule(tgvg_ctx* ctx, int n, int iters, bool stop, bool timed,
     int rc = iter_occupancy<MODE>(ctx), cmax = 0;
     if (!rc) rc = coop_capacity<MODE>(ctx, stop, &cmax);
     if (rc) return rc;
-    int tuned = ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, n))];
+    int* pick = nullptr;
+    if ((rc = tune_entry<MODE>(ctx, n, &pick))) return rc;
+    int tuned = *pick;
     if (tuned == CFG_FUSED_TMA && ctx->paged_now) tuned = CFG_FUSED;  // bulk copies stay on device-resident state
     if (timed) {  // per-launch event timing needs one of the per-sweep-launch or fused schedules
         *cfg = (per_launch_cfg(tuned) || ((fused_cfg(tuned) || wave_cfg(tuned)) && MODE != M_OC)) ? tuned : CFG_BAND;
@@ -3189,6 +3208,8 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
     if (cfg < 0) {
         std::vector<int> cands;
         if ((rc = tune_candidates<MODE>(ctx, a.n, cands))) return rc;
+        int* pick = nullptr;
+        if ((rc = tune_entry<MODE>(ctx, a.n, &pick))) return rc;
         float best_ms = 1e30f;
         int best = 0;
         const int ns = unit_slots<MODE>(a.nslot);
@@ -3209,7 +3230,7 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
                 bool all = true;
                 for (int d : done_h) all = all && d != 0;
                 if (all) {
-                    ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, a.n))] = best_ms < 1e30f ? best : c;
+                    *pick = best_ms < 1e30f ? best : c;
                     *used = effective_cfg<MODE>(ctx, c, a.n);
                     return TGVG_OK;
                 }
@@ -3219,7 +3240,7 @@ static int run_unit_t(tgvg_ctx* ctx, IterArgs& a, int iters, bool stop, bool tim
             ms /= (float)seg;
             if (ms < best_ms) { best_ms = ms; best = c; }
         }
-        ctx->tune[MODE][31 - __builtin_clz((unsigned)std::max(1, a.n))] = best;
+        *pick = best;
         cfg = best;
     }
     if (cfg == CFG_SMEM || cfg == CFG_REG) {
@@ -3601,7 +3622,8 @@ int tgv_solve_dev(tgvg_ctx* ctx, const tgvg_cube* d_cubes, const uint32_t* d_his
     // ---- wavefront-schedule tables, per level (in-memory and streaming semantics)
     std::vector<WaveSet> wsets(NBUCKET, WaveSet{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, false});
     bool wave_wanted = false;  // only a schedule set by tgvg_set_schedule runs it
-    for (int c : ctx->tune[mode]) wave_wanted |= wave_cfg(c);
+    for (const auto& c : ctx->tune[mode])
+        for (int k : c) wave_wanted |= wave_cfg(k);
     if (wave_wanted && mode != M_OC && fiters > 0 && n_act > 0) {
         const int rc = build_wave_tables(ctx, mode, min_d, max_d, h_bstart, n, nb, wsets);
         if (rc) return rc;

@@ -146,9 +146,15 @@ typedef struct tgvg_ctx tgvg_ctx;
 /* ---- context ---------------------------------------------------------------
  * One context per process and device: it owns the CUDA stream all calls run on
  * and a grow-only pool of device buffers reused across calls.  Calls on one
- * context are serialised by a mutex (the reference is single-threaded). */
+ * context are serialised by a mutex (the reference is single-threaded).  Besides
+ * that pool it keeps the scratch of merges and balances between calls: at most
+ * 8 GiB, or an eighth of the device budget where one is set
+ * (tgvg_set_device_budget).  tgvg_trim gives it back at once, for other users of
+ * the device's memory; the context itself does so before one of its own
+ * allocations fails. */
 int tgvg_create(int device, tgvg_ctx** out);
 int tgvg_destroy(tgvg_ctx* ctx);
+int tgvg_trim(tgvg_ctx* ctx);
 const char* tgvg_strerror(int rc);
 const char* tgvg_last_error(tgvg_ctx* ctx);
 int tgvg_abi_version(void);

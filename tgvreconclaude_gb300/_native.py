@@ -124,6 +124,7 @@ _SIGS = {
     "tgvg_abi_version": ([], C.c_int),
     "tgvg_create": ([C.c_int, C.POINTER(C.c_void_p)], C.c_int),
     "tgvg_destroy": ([P], C.c_int),
+    "tgvg_trim": ([P], C.c_int),
     "tgvg_strerror": ([C.c_int], C.c_char_p),
     "tgvg_last_error": ([P], C.c_char_p),
     "tgvg_stream": ([P], C.c_void_p),

@@ -54,6 +54,10 @@ class Context:
         """Fix the iteration schedule of a size class (tgvg_set_schedule)."""
         self.check(self.lib.tgvg_set_schedule(self.h, MODES[mode], cls, cfg), "tgvg_set_schedule")
 
+    def trim(self) -> None:
+        """Give the scratch kept between merges and balances back (tgvg_trim)."""
+        self.check(self.lib.tgvg_trim(self.h), "tgvg_trim")
+
     def kernel_count(self) -> int:
         return self.lib.tgvg_kernel_count(self.h)
 

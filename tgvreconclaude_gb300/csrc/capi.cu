@@ -34,8 +34,7 @@ void* tgvg_ctx::buf(int id, size_t bytes) {
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        ws_drop();
-        e = cudaMalloc(&b.p, bytes);
+        e = dev_alloc(&b.p, bytes);
         want = bytes;
     }
     if (e != cudaSuccess) {
@@ -101,13 +100,7 @@ void* tgvg_ctx::ws_get(size_t bytes) {
         return b.p;
     }
     Block b{nullptr, bytes};
-    cudaError_t e = cudaMalloc(&b.p, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        ws_drop();
-        e = cudaMalloc(&b.p, bytes);
-    }
-    if (e != cudaSuccess) {
+    if (dev_alloc(&b.p, bytes) != cudaSuccess) {
         cudaGetLastError();
         last_error = "cudaMalloc of " + std::to_string(bytes) + " bytes failed";
         return nullptr;
@@ -125,17 +118,25 @@ void tgvg_ctx::ws_put(void* p) {
             ws_idle_bytes += b.bytes;
             break;
         }
-    while (ws_idle_bytes > WS_CACHE_MAX && !ws_idle.empty()) {  // the oldest go first
+    ws_trim(ws_limit());
+}
+
+void tgvg_ctx::ws_trim(size_t limit) {
+    while (ws_idle_bytes > limit && !ws_idle.empty()) {
         ws_idle_bytes -= ws_idle.front().bytes;
         cudaFree(ws_idle.front().p);  // waits for its uses
         ws_idle.erase(ws_idle.begin());
     }
 }
 
-void tgvg_ctx::ws_drop() {
-    for (const Block& b : ws_idle) cudaFree(b.p);
-    ws_idle.clear();
-    ws_idle_bytes = 0;
+cudaError_t tgvg_ctx::dev_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ws_idle_bytes > 0) {
+        cudaGetLastError();
+        ws_drop();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 int tgvg_ctx::fail(int rc, const std::string& what) {
@@ -196,6 +197,14 @@ extern "C" int tgvg_set_device_budget(tgvg_ctx* ctx, int64_t bytes) {
     if (!ctx || bytes < 0) return TGVG_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->device_budget = (size_t)bytes;
+    ctx->ws_trim(ctx->ws_limit());
+    return TGVG_OK;
+}
+
+extern "C" int tgvg_trim(tgvg_ctx* ctx) {
+    if (!ctx) return TGVG_ERR_INVALID;
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    ctx->ws_drop();
     return TGVG_OK;
 }
 

@@ -229,14 +229,21 @@ struct tgvg_ctx {
     // device budget).  A buffer changes kind by being reallocated.
     void* host_backed(int id, size_t bytes);
     // Scratch blocks of calls whose sizes vary (merge, balance): taken from and
-    // given back to a cache of at most WS_CACHE_MAX bytes, all used on `stream`.
+    // given back to a cache, all used on `stream`.  At most ws_limit() bytes of
+    // it stay between calls: 8 GiB, or an eighth of the device budget.
     static constexpr size_t WS_CACHE_MAX = size_t(8) << 30;
+    size_t ws_limit() const {
+        return device_budget > 0 && device_budget / 8 < WS_CACHE_MAX ? device_budget / 8 : WS_CACHE_MAX;
+    }
     struct Block { void* p; size_t bytes; };
     std::vector<Block> ws_idle, ws_used;
     size_t ws_idle_bytes = 0;
     void* ws_get(size_t bytes);
     void ws_put(void* p);
-    void ws_drop();  // frees the idle blocks
+    void ws_trim(size_t limit);  // frees idle blocks, the oldest first, until at most `limit` bytes are idle
+    void ws_drop() { ws_trim(0); }
+    // cudaMalloc that gives the idle blocks back before it fails.
+    cudaError_t dev_alloc(void** p, size_t bytes);
     int fail(int rc, const std::string& what);
     int cuda_fail(cudaError_t e, const char* what);
 };

@@ -935,12 +935,13 @@ extern "C" int tgvg_mlp_create(tgvg_ctx* ctx, int32_t nbins, uint64_t seed, tgvg
     auto* m = new tgvg_mlp();
     m->nbins = nbins;
     float** bufs[] = {&m->d_prm, &m->d_m1, &m->d_m2, &m->d_grad, &m->d_wr};
-    for (float** b : bufs)
-        if (cudaMalloc(b, sizeof(float) * P_N) != cudaSuccess) { delete m; return TGVG_ERR_NOMEM; }
-    if (cudaMalloc(&m->d_loss, sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess ||
-        cudaMalloc(&m->d_tc, TC_W) != cudaSuccess) {
-        delete m;
+    bool ok = true;
+    for (float** b : bufs) ok = ok && ctx->dev_alloc((void**)b, sizeof(float) * P_N) == cudaSuccess;
+    if (!ok || ctx->dev_alloc((void**)&m->d_loss, sizeof(float)) != cudaSuccess ||
+        ctx->dev_alloc((void**)&m->d_frag, sizeof(uint32_t) * F_N) != cudaSuccess ||
+        ctx->dev_alloc((void**)&m->d_tc, TC_W) != cudaSuccess) {
+        cudaGetLastError();
+        tgvg_mlp_destroy(m);
         return TGVG_ERR_NOMEM;
     }
     // He-uniform weights over the real fan-in (the padded inputs stay zero), zero biases.

@@ -601,7 +601,8 @@ uint64_t pow2_at_least(uint64_t x) {
 
 // Device memory of one merge or balance run.  Blocks come from and go back to
 // the context's cache of such blocks (tgvg_ctx::ws_get / ws_put: at most
-// WS_CACHE_MAX bytes between calls, dropped when any allocation fails): a merge
+// ws_limit() bytes between calls, given back by tgvg_trim and before one of the
+// context's own allocations fails): a merge
 // made 9 and a balance about 30 cudaMalloc / cudaFree pairs per call, 0.9 ms of a
 // 2.8 ms merge and 4 ms of an 8.4 ms balance.  All uses of a block are on the
 // context's stream, so a block may be handed on while kernels still use it.

@@ -197,8 +197,8 @@ int tgvg_set_timing(tgvg_ctx* ctx, int on);
  * cubes), above that one cooperative launch over all SMs with the unit's state
  * in registers, or in shared memory and registers (units of at most about 3560
  * cubes per SM; larger units run 14), -1 = let the online autotuner choose (default),
- * once per class and on-chip kernel (23, 24's three) that holds the unit.  Results
- * do not depend on it. */
+ * once per class and on-chip kernel (23, 24's three) that holds the unit; it
+ * never chooses 1..6, 10, 11 or 20..22.  Results do not depend on it. */
 int tgvg_set_schedule(tgvg_ctx* ctx, int32_t mode, int32_t cls, int32_t cfg);
 /* CUDA graphs for the level loop (1 = on, the default; 0 = off).  When every
  * level's schedule is already fixed (chosen by the autotuner in an earlier

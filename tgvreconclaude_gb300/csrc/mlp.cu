@@ -350,12 +350,13 @@ __device__ __forceinline__ uint32_t pack_top(float a, float b) {
 //
 // Bytes: 16 + 4 NB read and 4 written per cube, 19 us for 2.2 M cubes of 10 bins;
 // what bounds it is the instructions of a row's features and its two epilogues
-// (about 650 a warp) and the latency between them.  Those cubes in 128 chunks:
+// (about 610 a warp) and the latency between them.  Those cubes in 128 chunks:
 // 104 us with mma.sync, at that instruction's 236 TFLOP/s, -> 93 us with tcgen05,
 // 78 us with the ReLU on packed pairs, neighbouring tiles and the prefetch, 77 us
 // with the weights copied as the products take them (k_mlp_pack lays them out when
 // they change; gathered from the FP32 parameters by each block, a call of 6,000 to
-// 600,000 cubes took 1.3 to 1.8 us longer: 17.6 and 36.5 us against 16.3 and 34.7).
+// 600,000 cubes took 1.3 to 1.8 us longer: 17.6 and 36.5 us against 16.3 and 34.7),
+// 75 us with the waits decided per warp.
 constexpr int TC_GROUPS = 8, TC_THREADS = TC_GROUPS * 128;
 constexpr int TC_CORE = 128 * 16;          // 128 rows x 8 columns
 constexpr int TC_A = 10 * TC_CORE;         // 80 columns: 64 activations, 3 ones, 13 zeros

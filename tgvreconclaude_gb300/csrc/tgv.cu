@@ -1370,7 +1370,10 @@ constexpr int SMEM_MAX_N = 2048;    // schedule 23 takes units of at most this m
 constexpr int REG_CTA_MAX = 1024;   // cubes (threads) per CTA
 // Schedule 23: cubes per CTA before another CTA is added.  A second CTA brings the
 // cluster barrier (0.6 us an iteration at one cube against 0.25), a full one the
-// issue slots of one SM; a 1,200-cube solve takes 847, 769 and 807 us at 128, 256 and 512.
+// issue slots of one SM.  us per iteration at 128, 256 and 512 cubes a CTA: units of
+// 200 cubes 0.90, 0.53, 0.53; 300: 0.99, 1.00, 0.65; 450: 1.01, 1.03, 0.75; 600: 0.98,
+// 1.02, 1.06; 900: 1.00, 1.05, 1.19; 1,200: 0.99, 0.99, 1.06; 1,600: 0.99, 0.99, 1.08;
+// 2,048: 1.00, 1.00, 1.14.  (One CTA up to 512 cubes would gain between 257 and 512.)
 constexpr int REG_CTA_AIM = 256;
 // bars and three face records per cube, a zero record, at most six staged records per cube
 static inline size_t reg_level_bytes(int chunk) { return 16 * (10 * size_t(chunk) + 1); }

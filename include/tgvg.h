@@ -198,7 +198,11 @@ int tgvg_set_timing(tgvg_ctx* ctx, int on);
  * in registers, or in shared memory and registers (units of at most about 3560
  * cubes per SM; larger units run 14), -1 = let the online autotuner choose (default),
  * once per class and on-chip kernel (23, 24's three) that holds the unit; it
- * never chooses 1..6, 10, 11 or 20..22.  Results do not depend on it. */
+ * never chooses 1..6, 10, 11 or 20..22.  Results do not depend on it.  1..6 and
+ * 24 above the cluster's size are cooperative launches, which start when all of
+ * their blocks have room: at 24 the largest need nearly all of every SM, so they
+ * wait for other streams' kernels to leave it.  A program that keeps a kernel
+ * resident on the GPU while it solves fixes 14, whose launches share it. */
 int tgvg_set_schedule(tgvg_ctx* ctx, int32_t mode, int32_t cls, int32_t cfg);
 /* CUDA graphs for the level loop (1 = on, the default; 0 = off).  When every
  * level's schedule is already fixed (chosen by the autotuner in an earlier
